@@ -10,20 +10,21 @@
 //     32 rows x 27 slots.  Inside a slice the slots are grouped per stencil
 //     z-plane (9 slots each) and, inside a plane, interleaved across the 32
 //     rows in short vectors: FP64 values in pairs of slots (one 16-byte load
-//     per row and pair), int32 columns and BF16 values in quads (one 16- or
-//     8-byte load), plus one single slot per plane.  A warp's load of one
-//     group for its 32 rows is one contiguous 512 / 256-byte segment, and a
-//     row needs 15 value loads and 9 column loads instead of 27 + 27;
+//     per row and pair), BF16 values in quads (one 8-byte load), plus one
+//     single slot per plane.  A warp's load of one group for its 32 rows is one
+//     contiguous 512 / 256-byte segment, and a row needs 15 (FP64) or 9 (BF16)
+//     value loads instead of 27;
 //   * slot s is the stencil offset (dz+1)*9 + (dy+1)*3 + (dx+1); slot 13 is the
-//     diagonal.  Absent neighbours (boundary rows) hold value 0 and column =
-//     the row itself.  Present entries therefore appear in exactly the
-//     (sz, sy, sx) order the reference generator emits
-//     (src/GenerateProblem_ref.cpp:152-172), which makes every row sum below
-//     round exactly as the reference's;
-//   * columns are int32 natural row indices, read by the FP64 sweeps and the
-//     plain solver's SpMV; the mixed V-cycle and the mixed solver's FP64 SpMV
-//     derive them from the stencil offsets instead (row + offset), so the
-//     BF16 copy holds values only; vectors stay in natural order.
+//     diagonal.  Absent neighbours (boundary rows) hold value 0.  Present
+//     entries therefore appear in exactly the (sz, sy, sx) order the reference
+//     generator emits (src/GenerateProblem_ref.cpp:152-172), which makes every
+//     row sum below round exactly as the reference's;
+//   * no column is stored: every loaded level is a 27-point stencil matrix (the
+//     loaders reject any other column), so slot s of a row is row + off[s]
+//     where that neighbour exists.  A stored int32 column would add 4 B to the
+//     8 B of an FP64 value in kernels that HBM bounds (set of 50 CG iterations
+//     at 256^3: 224 ms with stored columns, 185 ms without); vectors stay in
+//     natural order.
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -77,7 +78,6 @@ struct ClassInfo {
 template <class VT>
 struct LevelMat {
   const VT *vals;
-  const int32_t *cols;
   int nx, ny, nz;
   int64_t n;
   // z-slab halo planes present below / above (a neighbouring rank there), and
@@ -85,12 +85,13 @@ struct LevelMat {
   int zlo, zhi;
   int lo, span;
   int64_t srows;   // storage rows (colours padded to 32)
-  // Stencil offsets: slot s of row i holds column i + off[s] whenever the row
-  // has that neighbour (the layout enforces it when a level is loaded), and
-  // column i with value 0 otherwise.  The mixed-precision V-cycle and the
-  // mixed solver's SpMV derive their columns from these instead of reading
-  // `cols`.
+  // Stencil offsets: slot s of row i is column i + off[s] whenever the row has
+  // that neighbour (the layout enforces it when a level is loaded), and column
+  // i with value 0 otherwise.
   int off[HPCGX_STENCIL];
+  // a loaded matrix whose rows leave out entries of existing neighbours: such a
+  // slot (value 0) is column i too
+  int holes;
 };
 
 // Elements of one 32-row slice and of one z-plane inside it.
@@ -105,8 +106,8 @@ __host__ __device__ inline int64_t vidx(int64_t k, int s) {
   const int lane = (int)(k & 31);
   return r < 8 ? base + (r >> 1) * 64 + lane * 2 + (r & 1) : base + 256 + lane;
 }
-// Index of (storage row k, slot s) in the column and BF16 value arrays: per
-// plane, slots r = 0..7 in interleaved quads, slot r = 8 alone.
+// Index of (storage row k, slot s) in the BF16 value array: per plane, slots
+// r = 0..7 in interleaved quads, slot r = 8 alone.
 __host__ __device__ inline int64_t cidx(int64_t k, int s) {
   const int p = s / 9, r = s - 9 * p;
   const int64_t base = (k >> 5) * kSliceElems + p * kPlaneElems;

@@ -263,7 +263,6 @@ __device__ __forceinline__ int64_t check_index(int64_t i, int64_t n, int site) {
 
 struct ClassSet {
   ClassInfo c[4];
-  int lpb[4];      // lines per block
   int nblk[4];     // blocks of each class
   int common;      // min over the classes of nblk
   int total;       // sum of nblk: the grid
@@ -326,22 +325,6 @@ __device__ __forceinline__ void check_cols(const LevelMat<VT> &A, int32_t *col, 
 #endif
 }
 
-__device__ __forceinline__ RowId row_of(const ClassInfo &C, int nx, int ny, int px, int j0,
-                                        int t) {
-  const int Lp = C.len[px];
-  const int jl = (int)fdiv((uint32_t)t, C.dlen[px]);
-  const int pos = t - jl * Lp;
-  const int j = j0 + jl;
-  const int jz = (int)fdiv((uint32_t)j, C.dnyq);
-  RowId r;
-  r.iy = C.py + 2 * (j - jz * C.nyq);
-  r.iz = C.pz + 2 * jz;
-  r.ix = px + 2 * pos;
-  r.row = ((int64_t)r.iz * ny + r.iy) * nx + r.ix;
-  r.k = C.start[px] + (int64_t)j * Lp + pos;
-  return r;
-}
-
 // ---------------------------------------------------------------- row loads
 
 // Vector loads of one stencil z-plane (9 slots) of storage row k; a group is
@@ -382,25 +365,6 @@ __device__ __forceinline__ void load_plane(const uint16_t *__restrict__ vals, in
   if (need(9 * p + 8)) v[8] = __ldg(q + 256 + lane);
 }
 
-template <class NEED>
-__device__ __forceinline__ void load_plane(const int32_t *__restrict__ cols, int64_t k, int p,
-                                           NEED need, int32_t *c) {
-  const int32_t *q = cols + (k >> 5) * kSliceElems + p * kPlaneElems;
-  const int lane = (int)(k & 31);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    if (need(9 * p + 4 * j) || need(9 * p + 4 * j + 1) || need(9 * p + 4 * j + 2) ||
-        need(9 * p + 4 * j + 3)) {
-      const int4 t = __ldg(reinterpret_cast<const int4 *>(q + j * 128 + lane * 4));
-      c[4 * j] = t.x;
-      c[4 * j + 1] = t.y;
-      c[4 * j + 2] = t.z;
-      c[4 * j + 3] = t.w;
-    }
-  }
-  if (need(9 * p + 8)) c[8] = __ldg(q + 256 + lane);
-}
-
 // BF16 values of one z-plane straight to FP32 (a BF16 pattern is the high
 // half of the FP32 pattern of the same number).
 template <class NEED>
@@ -432,100 +396,234 @@ __device__ __forceinline__ void load_vals(const uint16_t *__restrict__ vals, int
   load_plane_f32(vals, k, p, need, v);
 }
 
+// The values of one row in registers: FP64 as they are; BF16 packed as loaded
+// (15 registers a row instead of 27) and widened where they are used.
+template <class VT>
+struct RowVals;
+template <>
+struct RowVals<double> {
+  double v[HPCGX_STENCIL];
+  template <class NEED>
+  __device__ __forceinline__ void load(const double *vals, int64_t k, int p, NEED need) {
+    load_plane(vals, k, p, need, v + 9 * p);
+  }
+  __device__ __forceinline__ double get(int s) const { return v[s]; }
+};
+template <>
+struct RowVals<uint16_t> {
+  uint2 q[6];
+  uint32_t one[3];
+  template <class NEED>
+  __device__ __forceinline__ void load(const uint16_t *vals, int64_t k, int p, NEED need) {
+    const uint16_t *w = vals + (k >> 5) * kSliceElems + p * kPlaneElems;
+    const int lane = (int)(k & 31);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (need(9 * p + 4 * j) || need(9 * p + 4 * j + 1) || need(9 * p + 4 * j + 2) ||
+          need(9 * p + 4 * j + 3))
+        q[2 * p + j] = __ldg(reinterpret_cast<const uint2 *>(w + j * 128 + lane * 4));
+    if (need(9 * p + 8)) one[p] = __ldg(w + 256 + lane);
+  }
+  // a BF16 pattern is the high half of the FP32 pattern of the same number
+  __device__ __forceinline__ float get(int s) const {
+    const int p = s / 9, i = s % 9;
+    if (i == 8) return __uint_as_float(one[p] << 16);
+    const uint2 t = q[2 * p + i / 4];
+    const uint32_t w = (i % 4) < 2 ? t.x : t.y;
+    return (i & 1) ? __uint_as_float(w & 0xffff0000u) : __uint_as_float(w << 16);
+  }
+};
+
 struct NeedAll {
   __device__ constexpr bool operator()(int) const { return true; }
 };
 
-// ---------------------------------------------------------------- SpMV
+// ---------------------------------------------------------------- columns
 
-// Columns of storage row id derived from the stencil offsets, row + off[s] in
-// 32-bit arithmetic (vectors hold fewer than 2^31 rows).  Every level matrix
-// is a 27-point stencil matrix (the loaders reject any other pattern) whose
-// absent neighbours hold the value 0 and the row itself as column, so the
-// stored int32 columns carry no information: an interior row reads exactly
-// row + off[s].  A slot of a boundary row without a neighbour multiplies its
-// x entry by 0.  EXACT takes the row itself for every such slot, as the
-// stored columns do: the Gauss-Seidel sweeps need it, since another block of
-// the same launch may write some rows for the first time (x there may hold
-// anything, NaN included) while this row's own entry is written already, and
-// it also keeps their gathers on lines the row reads anyway.  The SpMV reads
-// a fully written x, where any entry serves: it keeps row + off[s] where that
-// lies inside the vector and takes the row itself elsewhere (one compare per
-// slot, fewer instructions than the exact test).
-template <bool EXACT, class VT, class NEED>
-__device__ __forceinline__ void stencil_cols(const LevelMat<VT> &A, const RowId &id, NEED need,
+// Columns of storage row id: row + off[s] where that neighbour exists (in
+// 32-bit arithmetic: vectors hold fewer than 2^31 rows), the row itself
+// elsewhere and for a left-out entry, so that the product with the slot's 0
+// reads nothing the row does not read anyway.
+template <class VT, class V>
+__device__ __forceinline__ void stencil_cols(const LevelMat<VT> &A, const RowId &id, const V *val,
                                              int32_t *col) {
   const int r32 = (int)id.row;
   const bool xm = id.ix > 0, xp = id.ix + 1 < A.nx, ym = id.iy > 0, yp = id.iy + 1 < A.ny,
              zm = id.iz > 0 || A.zlo, zp = id.iz + 1 < A.nz || A.zhi;
-  if (xm && xp && ym && yp && zm && zp) {
 #pragma unroll
-    for (int s = 0; s < HPCGX_STENCIL; ++s)
-      if (need(s)) col[s] = r32 + A.off[s];
-  } else if (EXACT) {
-#pragma unroll
-    for (int s = 0; s < HPCGX_STENCIL; ++s)
-      if (need(s)) {
-        const int dx = s % 3 - 1, dy = (s / 3) % 3 - 1, dz = s / 9 - 1;
-        const bool nb = (dx < 0 ? xm : dx > 0 ? xp : true) && (dy < 0 ? ym : dy > 0 ? yp : true) &&
-                        (dz < 0 ? zm : dz > 0 ? zp : true);
-        col[s] = nb ? r32 + A.off[s] : r32;
-      }
-  } else {
-#pragma unroll
-    for (int s = 0; s < HPCGX_STENCIL; ++s)
-      if (need(s)) {
-        const int cc = r32 + A.off[s];
-        col[s] = (uint32_t)(cc - A.lo) < (uint32_t)A.span ? cc : r32;
-      }
+  for (int s = 0; s < HPCGX_STENCIL; ++s) {
+    const int dx = s % 3 - 1, dy = (s / 3) % 3 - 1, dz = s / 9 - 1;
+    const bool nb = (dx < 0 ? xm : dx > 0 ? xp : true) && (dy < 0 ? ym : dy > 0 ? yp : true) &&
+                    (dz < 0 ? zm : dz > 0 ? zp : true) && !(A.holes && val[s] == V(0));
+    col[s] = nb ? r32 + A.off[s] : r32;
   }
 }
 
+// ---------------------------------------------------------------- row pairs
+
+// SpMV and the sweeps give a thread the two rows (2i, 2i+1) of an x-line.  On
+// each of the 9 stencil lines (dy, dz) both rows read x[2i-1 .. 2i+2] between
+// them, so a pair gathers 9 x 4 entries with 27 loads (two entries in one
+// vector load) instead of 54, from 9 line addresses instead of 54.
+struct PairId {
+  int64_t row;      // natural index of the even row
+  int64_t ke, ko;   // storage rows
+  int ix, iy, iz;   // of the even row
+  int pos;          // pair inside its line
+  bool left, odd, right;   // x-neighbours of the even row at -1, +1, +2 exist
+  bool ym, yp, zm, zp;     // the lines below / above exist
+};
+
+template <class VT>
+__device__ __forceinline__ PairId pair_of(const LevelMat<VT> &A, const ClassInfo &C, int j0, int t,
+                                          int site) {
+  PairId id;
+  const int Le = C.len[0];
+  const int jl = (int)fdiv((uint32_t)t, C.dlen[0]);
+  id.pos = t - jl * Le;
+  const int j = j0 + jl;
+  const int jz = (int)fdiv((uint32_t)j, C.dnyq);
+  id.iy = C.py + 2 * (j - jz * C.nyq);
+  id.iz = C.pz + 2 * jz;
+  id.ix = 2 * id.pos;
+  id.row = ((int64_t)id.iz * A.ny + id.iy) * A.nx + id.ix;
+  id.ke = C.start[0] + (int64_t)j * Le + id.pos;
+  id.ko = C.start[1] + (int64_t)j * C.len[1] + id.pos;
+  id.left = id.pos > 0;
+  id.odd = id.pos < C.len[1];
+  id.right = id.pos + 1 < Le;
+  id.ym = id.iy > 0;
+  id.yp = id.iy + 1 < A.ny;
+  id.zm = id.iz > 0 || A.zlo;
+  id.zp = id.iz + 1 < A.nz || A.zhi;
+  if (!id.odd) id.ko = id.ke;
+#ifdef HPCGX_CHECKED
+  if (id.row < 0 || id.row + (id.odd ? 1 : 0) >= A.n) {
+    check_fail(site, id.row);
+    id.row = 0;
+  }
+  if (id.ke < 0 || id.ke >= A.srows || id.ko < 0 || id.ko >= A.srows) {
+    check_fail(site, id.ke);
+    id.ke = id.ko = 0;
+  }
+#endif
+  return id;
+}
+
+// Stencil line l = (dz+1)*3 + (dy+1): does it exist for the pair's rows?
+__device__ __forceinline__ bool has_line(const PairId &id, int l) {
+  const int dy = l % 3 - 1, dz = l / 3 - 1;
+  return (dy < 0 ? id.ym : dy > 0 ? id.yp : true) && (dz < 0 ? id.zm : dz > 0 ? id.zp : true);
+}
+
+__device__ __forceinline__ void load2(const double *p, double &u, double &v) {
+  const double2 t = *reinterpret_cast<const double2 *>(p);
+  u = t.x;
+  v = t.y;
+}
+__device__ __forceinline__ void load2(const float *p, float &u, float &v) {
+  const float2 t = *reinterpret_cast<const float2 *>(p);
+  u = t.x;
+  v = t.y;
+}
+__device__ __forceinline__ void store2(double *p, double u, double v) {
+  *reinterpret_cast<double2 *>(p) = make_double2(u, v);
+}
+__device__ __forceinline__ void store2(float *p, float u, float v) {
+  *reinterpret_cast<float2 *>(p) = make_float2(u, v);
+}
+
+// x[2i-1 .. 2i+2] on line l into v[0..3]; what does not exist (or is not on)
+// reads as 0, the value its slots hold, so that the product drops out whatever
+// x holds elsewhere.  vec: the two middle entries with one load (x and nx allow it).
+template <class VT, class T>
+__device__ __forceinline__ void load_line(const LevelMat<VT> &A, const PairId &id, const T *xr,
+                                          int l, bool on, bool vec, T *v, int site) {
+  const bool ok = on && has_line(id, l);
+  const T *q = xr + A.off[3 * l + 1];
+#ifdef HPCGX_CHECKED
+  const int64_t at = id.row + A.off[3 * l + 1];
+  if (ok && ((at - (id.left ? 1 : 0) - A.lo) < 0 ||
+             (at + (id.right ? 2 : id.odd ? 1 : 0) - A.lo) >= A.span)) {
+    check_fail(site, at);
+    q = xr - id.row + 1;
+  }
+#endif
+  v[0] = v[1] = v[2] = v[3] = T(0);
+  if (ok && id.left) v[0] = q[-1];
+  if (vec) {
+    if (ok) load2(q, v[1], v[2]);
+  } else {
+    if (ok) v[1] = q[0];
+    if (ok && id.odd) v[2] = q[1];
+  }
+  if (ok && id.right) v[3] = q[2];
+}
+
+// One term of a row sum.  holes: a left-out entry (value 0) adds nothing
+// whatever its neighbour holds (LevelMat::holes).
+template <class T>
+__device__ __forceinline__ T term_add(bool holes, T sum, T v, T x) {
+  return holes && v == T(0) ? sum : mac_add(sum, v, x);
+}
+template <class T>
+__device__ __forceinline__ T term_sub(bool holes, T sum, T v, T x) {
+  return holes && v == T(0) ? sum : mac_sub(sum, v, x);
+}
+
+// ---------------------------------------------------------------- SpMV
+
 // y = A x, rows summed left to right over the slots as ComputeSPMV_ref does
 // (src/ComputeSPMV_ref.cpp:64-70).  With DOT, also reduces sum_i x_i y_i (the
-// p.Ap of CG, src/CG.cpp:119) and runs the finishing scalar step.  IMPL
-// derives the columns from the stencil offsets instead of reading them.
-// Occupancy: with stored columns a row keeps 54 loads in flight and two
-// blocks per SM saturate HBM; without column loads the gathers issue at once
-// and three blocks per SM (80 registers) hide their latency best (measured at
-// 512^3: 4.60 ms against 5.06 ms at four blocks and 5.80 ms at five).
-template <bool IMPL>
-constexpr int spmv_min_blocks() { return IMPL ? 3 : 2; }
-
-template <class VT, class T, bool DOT, bool IMPL>
-__global__ void __launch_bounds__(kThreads, spmv_min_blocks<IMPL>())
-k_spmv(LevelMat<VT> A, ClassSet cs, const T *__restrict__ x, T *__restrict__ y, Reduce red,
-       int fin, void *fin_target, const int *__restrict__ done) {
+// p.Ap of CG, src/CG.cpp:119) and runs the finishing scalar step.  A block
+// takes 256 consecutive pairs of one class, whatever lines they lie on (rows
+// have no order to keep), so no thread idles on ragged lines; the classes are
+// interleaved block by block (class_block).  HBM bounds it: 8 B per nonzero and
+// 16 B per row at 256^3 is 3.86 GB, 568 us = 6.8 TB/s, 1.04 of the measured
+// copy rate (one row per thread and stored int32 columns: 824 us; 104^3: 59
+// against 78 us).  FP64 holds a z-plane's 18 values and 12 entries per step
+// (128 registers, two blocks per SM); one and three blocks measured the same.
+template <class VT, class T, bool DOT, bool GEN>
+__global__ void __launch_bounds__(kThreads, std::is_same<VT, double>::value ? 2 : 4)
+k_spmv(LevelMat<VT> A, ClassSet cs, const T *__restrict__ x, T *__restrict__ y, int wide,
+       Reduce red, int fin, void *fin_target, const int *__restrict__ done) {
   if (done && *done) return;
+  const bool vec = !GEN || wide, holes = GEN && A.holes;
   int q, b;
   class_block(cs, (int)blockIdx.x, q, b);
   const ClassInfo &C = cs.c[q];
-  const int j0 = b * cs.lpb[q];
-  const int j1 = min(j0 + cs.lpb[q], C.lines);
+  const int t = b * kThreads + (int)threadIdx.x;
   double acc = 0.0;
-  for (int px = 0; px < 2; ++px) {
-    const int cnt = (j1 - j0) * C.len[px];
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-      RowId id = row_of(C, A.nx, A.ny, px, j0, t);
-      check_row(A, id, 1);
-      int32_t col[HPCGX_STENCIL];
-      VT val[HPCGX_STENCIL];
+  if (t < C.lines * C.len[0]) {
+    const PairId id = pair_of(A, C, 0, t, 1);
+    const T *xr = x + id.row;
+    T se = T(0), so = T(0), xe = T(0), xo = T(0);
 #pragma unroll
-      for (int p = 0; p < 3; ++p) {
-        if (!IMPL) load_plane(A.cols, id.k, p, NeedAll(), col + 9 * p);
-        load_plane(A.vals, id.k, p, NeedAll(), val + 9 * p);
+    for (int p = 0; p < 3; ++p) {
+      T ve[9], vo[9], v[3][4];
+      load_vals(A.vals, id.ke, p, NeedAll(), ve);
+      load_vals(A.vals, id.ko, p, NeedAll(), vo);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) load_line(A, id, xr, 3 * p + i, true, vec, v[i], 2);
+#pragma unroll
+      for (int s = 0; s < 9; ++s) {
+        se = term_add(holes, se, ve[s], v[s / 3][s % 3]);
+        so = term_add(holes, so, vo[s], v[s / 3][s % 3 + 1]);
       }
-      if (IMPL) stencil_cols<false>(A, id, NeedAll(), col);
-      check_cols(A, col, NeedAll(), 2);
-      T xv[HPCGX_STENCIL];
-#pragma unroll
-      for (int s = 0; s < HPCGX_STENCIL; ++s) xv[s] = __ldg(x + col[s]);
-      T sum = T(0);
-#pragma unroll
-      for (int s = 0; s < HPCGX_STENCIL; ++s) sum = mac_add(sum, to_arith(val[s], T()), xv[s]);
-      const T xrow = xv[HPCGX_DIAG_SLOT];
-      y[id.row] = sum;
-      if (DOT) acc += (double)xrow * (double)sum;
+      if (p == 1) {
+        xe = v[1][1];
+        xo = v[1][2];
+      }
+    }
+    if (vec && id.odd) {
+      store2(y + id.row, se, so);
+    } else {
+      y[id.row] = se;
+      if (id.odd) y[id.row + 1] = so;
+    }
+    if (DOT) {
+      acc = (double)xe * (double)se;
+      if (id.odd) acc += (double)xo * (double)so;
     }
   }
   if (DOT) {
@@ -540,190 +638,230 @@ k_spmv(LevelMat<VT> A, ClassSet cs, const T *__restrict__ x, T *__restrict__ y, 
 // One Gauss-Seidel row update, src/ComputeSYMGS_ref.cpp:72-80:
 //   sum = r_i - sum_j a_ij x_j (diagonal included, slot order); sum += x_i a_ii;
 //   x_i = sum / a_ii.
-// The loads are issued in three stages (every column and value, then every
-// neighbour of x, then the arithmetic) so that a thread keeps ~54 independent
-// loads in flight instead of walking a chain of dependent ones.
-// ZERO: x is known to be zero for every colour above c and for row i itself
-//       (first forward sweep after ZeroVector); those terms, and the padding
-//       slots (column = row), are skipped.  Skipping a product with a zero
-//       changes nothing but possibly the sign of an exact zero.
-// PRO:  x_i first receives the prolongated coarse correction (colour 0) --
-//       except in the first plane of a slab with a halo below, whose
-//       correction is added before the halo exchange (the slab below reads
-//       that plane).
-// RES:  after the update, the fine residual at this injected point is formed
-//       and restricted: rc = r_i - (A x)_i with (A x)_i summed as in SpMV.
-//       (A slab with a halo below forms its first plane's again once the
-//       halo holds the slab below's smoothed values.)
-// SYM:  forward update of a row of the last colour, immediately followed by
-//       its backward update (the first step of the backward sweep): between
-//       the two only x_i changes, so the backward value is recomputed from the
-//       same registers and only that value is stored.
-template <bool ZERO, bool PRO, bool RES, bool SYM = false, bool STN = false, class VT, class T,
-          class RT>
-__device__ __forceinline__ void gs_row(const LevelMat<VT> &A, const RowId &id0, int c,
-                                       const RT *__restrict__ r, T *x, const T *__restrict__ xc,
-                                       T *__restrict__ rc) {
-  RowId id = id0;
-  check_row(A, id, 3);
-  int32_t col[HPCGX_STENCIL];
-  T val[HPCGX_STENCIL];   // values converted to the arithmetic type as loaded
-  // slots whose neighbour is read: all, or (zero guess) the lower colours
-  auto need = [c](int s) { return !ZERO || s == HPCGX_DIAG_SLOT || ((c ^ slot_mask(s)) < c); };
-  // The mixed V-cycle (BF16 values) derives its columns from the stencil
-  // offsets; the FP64 path reads the stored int32 columns, or derives them
-  // too (STN, the FP64 solve with stencil columns).
-  constexpr bool IMPLICIT = STN || std::is_same<VT, uint16_t>::value;
+// The terms are taken in two parts: the slots of the stencil lines 0 .. 3
+// (slots 0 .. 11), and those of line 4, the row's own, and lines 5 .. 8.  Only
+// the own line changes while a class is swept, so the first part is summed as
+// soon as it is loaded -- once for a row that is updated twice (class 3) and
+// for the residual that GS_RESTRICT forms -- and only the second part stays in
+// registers over the exchange between the two rows of a pair.
+// PX: the row's place in the pair (0 even, 1 odd); c: its colour.
+// ZERO: x is zero for every colour above c and for the row itself (first
+//       forward sweep after ZeroVector); those terms are skipped.  Skipping a
+//       product with a zero changes nothing but possibly the sign of an exact
+//       zero.
+constexpr int kHead = 12;   // slots of the first part
+
+template <int PX, bool ZERO, class V, class T>
+__device__ __forceinline__ T gs_head(bool holes, int c, const V &val, const T (&xl)[4][4], T sum) {
 #pragma unroll
-  for (int p = 0; p < 3; ++p) {
-    load_vals(A.vals, id.k, p, need, val + 9 * p);
-    if (!IMPLICIT) load_plane(A.cols, id.k, p, need, col + 9 * p);
-  }
-  if (IMPLICIT) stencil_cols<true>(A, id, need, col);
-  check_cols(A, col, need, 4);
-  const T rhs = vec_to(__ldg(r + id.row), T());
-  int64_t crow = 0;
-  if (PRO || RES) {
-    const int nxc = A.nx >> 1, nyc = A.ny >> 1;
-    crow = ((int64_t)(id.iz >> 1) * nyc + (id.iy >> 1)) * nxc + (id.ix >> 1);
-    crow = check_index(crow, (int64_t)nxc * nyc * (A.nz >> 1), 5);
-  }
-  T xi = ZERO ? T(0) : x[id.row];
-  if (PRO && !(A.zlo && id.iz == 0)) xi = rn_add(xi, __ldg(xc + crow));
-  // A slot without a neighbour holds value 0 and the row itself as column; in
-  // the zero-guess sweep x_i is unwritten, so that term -- a product with 0 --
-  // is skipped below.  The gather itself does not wait for the value: every
-  // column is in range.
-  T xv[HPCGX_STENCIL];
+  for (int s = 0; s < kHead; ++s)
+    if (!(ZERO && (c ^ slot_mask(s)) > c))
+      sum = term_sub(holes, sum, (T)val.get(s), xl[s / 3][s % 3 + PX]);
+  return sum;
+}
+
+// xl[l - 4][0..3] = x[2i-1 .. 2i+2] of line l; xi: the row's own entry before
+// the update.
+template <int PX, bool ZERO, class V, class T>
+__device__ __forceinline__ T gs_tail(bool holes, int c, const V &val, const T (&xl)[5][4], T sum, T xi) {
+  const T d = val.get(HPCGX_DIAG_SLOT);
 #pragma unroll
-  for (int s = 0; s < HPCGX_STENCIL; ++s) {
-    if (s == HPCGX_DIAG_SLOT) continue;
-    if (ZERO && ((c ^ slot_mask(s)) > c)) continue;
-    xv[s] = x[col[s]];
-  }
-  T sum = rhs;
-  const T d = val[HPCGX_DIAG_SLOT];
-#pragma unroll
-  for (int s = 0; s < HPCGX_STENCIL; ++s) {
+  for (int s = kHead; s < HPCGX_STENCIL; ++s) {
     if (s == HPCGX_DIAG_SLOT) {
       if (!ZERO) sum = mac_sub(sum, d, xi);
-      continue;
+    } else if (!(ZERO && (c ^ slot_mask(s)) > c)) {
+      sum = term_sub(holes, sum, (T)val.get(s), xl[s / 3 - 4][s % 3 + PX]);
     }
-    if (ZERO && (((c ^ slot_mask(s)) > c) || val[s] == T(0))) continue;
-    sum = mac_sub(sum, val[s], xv[s]);
   }
   if (!ZERO) sum = mac_add(sum, xi, d);
-  const T xn = rn_div(sum, d);
-  if (SYM) {
-    T sum2 = rhs;
-#pragma unroll
-    for (int s = 0; s < HPCGX_STENCIL; ++s) {
-      if (s == HPCGX_DIAG_SLOT) {
-        sum2 = mac_sub(sum2, d, xn);
-        continue;
+  return rn_div(sum, d);
+}
+
+// A half sweep of one class over its lines [j0, j1), by one block: colours ce
+// then ce + 1 (DIR = 0) or ce + 1 then ce (DIR = 1), ce = 2 C.q.  A thread
+// updates both rows of a pair; the colours of a class only depend on each
+// other along x inside a line, and the block owns whole lines, so the entry
+// that the second row needs from the next pair (the next even one forward, the
+// previous odd one backward) comes through shared memory, and every load of
+// the pair was issued before the first update.
+// ZERO: x is zero for the colours above and for the row itself (first forward
+//       sweep after ZeroVector); their terms are skipped at compile time.
+//       zero: the same at run time, those entries read as 0.
+// pro:  colour 0 first receives the prolongated coarse correction -- except in
+//       the first plane of a slab with a halo below, whose correction is added
+//       before the halo exchange (the slab below reads that plane).
+// res:  after its update, the fine residual at the injected points (colour 0)
+//       is formed and restricted: rc = r_i - (A x)_i with (A x)_i summed as in
+//       SpMV (a slab with a halo below forms its first plane's again once the
+//       halo holds the slab below's smoothed values).
+// SYM3: forward and backward half sweep of the last class (DIR = 0): colour 6
+//       forward, colour 7 forward and backward, colour 6 backward.
+// Lines longer than a block are taken in chunks of blockDim pairs, from right
+// to left forward and from left to right backward: a chunk then finds the
+// neighbours that its first row must see unchanged unchanged, and those that
+// its second row must see updated updated.
+template <int DIR, bool ZERO, bool SYM3, class VT, class T, class RT>
+__device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo &C, int ce, int j0,
+                                         int j1, bool zero, bool pro, bool res, bool vec,
+                                         bool holes, const RT *r, T *x, const T *xc, T *rc, T *sh) {
+  const int cnt = (j1 - j0) * C.len[0];
+  const int nb = blockDim.x, tid = threadIdx.x;
+  const int chunks = (cnt + nb - 1) / nb;
+  const int co = ce + 1;
+  // a value is read if its slot is: all, or (ZERO) those of the lower colours
+  auto need_e = [=](int s) { return !ZERO || SYM3 || s == HPCGX_DIAG_SLOT || (ce ^ slot_mask(s)) < ce; };
+  auto need_o = [=](int s) { return !ZERO || s == HPCGX_DIAG_SLOT || (co ^ slot_mask(s)) < co; };
+  for (int ch = 0; ch < chunks; ++ch) {
+    if (ch) __syncthreads();   // the chunk before has stored its rows and read sh
+    const int t = (DIR == 0 ? chunks - 1 - ch : ch) * nb + tid;
+    const bool act = t < cnt;
+    PairId id;
+    RowVals<VT> ve, vo;
+    T xl[5][4];
+    T se = T(0), so = T(0), ax = T(0), xe = T(0), xo = T(0), re = T(0);
+    int64_t crow = 0;
+    if (act) {
+      id = pair_of(A, C, j0, t, 3);
+      const T *xr = x + id.row;
+      T ro = T(0);
+      if (vec) {
+        RT u, v;
+        load2(r + id.row, u, v);
+        re = vec_to(u, T());
+        ro = vec_to(v, T());
+      } else {
+        re = vec_to(r[id.row], T());
+        if (id.odd) ro = vec_to(r[id.row + 1], T());
       }
-      if (val[s] == T(0)) continue;   // a product with 0: no change
-      sum2 = mac_sub(sum2, val[s], xv[s]);
-    }
-    sum2 = mac_add(sum2, xn, d);
-    x[id.row] = rn_div(sum2, d);
-    return;
-  }
-  x[id.row] = xn;
-  if (RES) {
-    T ax = T(0);
+      {
+        T xh[4][4];
 #pragma unroll
-    for (int s = 0; s < HPCGX_STENCIL; ++s)
-      ax = mac_add(ax, val[s], s == HPCGX_DIAG_SLOT ? xn : xv[s]);
-    rc[crow] = rn_sub(rhs, ax);
-  }
-}
-
-// One half sweep of class Q over the lines [j0, j1) of the class: colours
-// 2Q then 2Q+1 (DIR = 0) or 2Q+1 then 2Q (DIR = 1).  A block owns whole lines,
-// so the x-neighbours of a row (the other colour of the class) are its own.
-// PRO / RES act on colour 0 only.
-template <int MODE, int Q, int DIR, class VT, class T, class RT>
-__device__ __forceinline__ void gs_lines(const LevelMat<VT> &A, const ClassInfo &C, int j0, int j1,
-                                         const RT *__restrict__ r, T *x,
-                                         const T *__restrict__ xc, T *__restrict__ rc) {
-  constexpr bool ZERO = (MODE & GS_ZERO_GUESS) != 0, PRO = (MODE & GS_PROLONG) != 0,
-                 RES = (MODE & GS_RESTRICT) != 0, STN = (MODE & GS_STENCIL) != 0;
+        for (int p = 0; p < 3; ++p) {
+          ve.load(A.vals, id.ke, p, need_e);
+          vo.load(A.vals, id.ko, p, need_o);
+        }
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int px = DIR ? 1 - half : half;
-    const int c = px + 2 * (Q >= 0 ? Q : C.q);
-    const int cnt = (j1 - j0) * C.len[px];
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-      const RowId id = row_of(C, A.nx, A.ny, px, j0, t);
-      if ((PRO || RES) && c == 0)
-        gs_row<ZERO, PRO, RES, false, STN>(A, id, c, r, x, xc, rc);
-      else
-        gs_row<ZERO, false, false, false, STN>(A, id, c, r, x, xc, rc);
+        for (int l = 0; l < 9; ++l) {
+          T *to = l < 4 ? xh[l < 4 ? l : 0] : xl[l < 4 ? 0 : l - 4];
+          // in the zero-guess sweep the pair's own line and those of the higher
+          // classes are not written yet
+          const bool there = l != 4 && (ce ^ (slot_mask(3 * l + 1))) < ce;
+          if (ZERO && !there)
+            to[0] = to[1] = to[2] = to[3] = T(0);
+          else
+            load_line(A, id, xr, l, !zero || there, vec, to, 4);
+        }
+        se = gs_head<0, ZERO>(holes, ce, ve, xh, re);
+        so = gs_head<1, ZERO>(holes, co, vo, xh, ro);
+        if (res) {
+#pragma unroll
+          for (int s = 0; s < kHead; ++s) ax = term_add(holes, ax, (T)ve.get(s), xh[s / 3][s % 3]);
+        }
+      }
+      if (pro || res) {
+        const int nxc = A.nx >> 1, nyc = A.ny >> 1;
+        crow = ((int64_t)(id.iz >> 1) * nyc + (id.iy >> 1)) * nxc + id.pos;
+        crow = check_index(crow, (int64_t)nxc * nyc * (A.nz >> 1), 5);
+      }
+      xe = xl[0][1];
+      xo = xl[0][2];
+      if (pro && !(A.zlo && id.iz == 0)) xe = rn_add(xe, xc[crow]);
+      if (DIR == 0) {
+        xe = gs_tail<0, ZERO>(holes, ce, ve, xl, se, xe);
+        sh[tid] = xe;
+      } else if (id.odd) {
+        xo = gs_tail<1, false>(holes, co, vo, xl, so, xo);
+        sh[tid + 1] = xo;
+      }
     }
-    if (half == 0) __syncthreads();
+    __syncthreads();
+    if (act) {
+      if (DIR == 0) {
+        xl[0][1] = xe;
+        if (id.right) xl[0][3] = tid + 1 < nb ? sh[tid + 1] : x[id.row + 2];
+        if (id.odd) {
+          xo = gs_tail<1, ZERO>(holes, co, vo, xl, so, xo);
+          // forward then backward: between the two only the row's own entry
+          // changes
+          if (SYM3) xo = gs_tail<1, false>(holes, co, vo, xl, so, xo);
+        }
+      } else {
+        xl[0][2] = xo;
+        if (id.left) xl[0][0] = tid > 0 ? sh[tid] : x[id.row - 1];
+        xe = gs_tail<0, false>(holes, ce, ve, xl, se, xe);
+      }
+      if (res) {
+#pragma unroll
+        for (int s = kHead; s < HPCGX_STENCIL; ++s)
+          ax = term_add(holes, ax, (T)ve.get(s),
+                               s == HPCGX_DIAG_SLOT ? xe : xl[s / 3 - 4][s % 3]);
+        rc[crow] = rn_sub(re, ax);
+      }
+    }
+    if (SYM3 && chunks == 1) {
+      __syncthreads();
+      if (act) sh[tid + 1] = xo;
+      __syncthreads();
+      if (act) {
+        xl[0][2] = xo;
+        if (id.left) xl[0][0] = sh[tid];
+        xe = gs_tail<0, false>(holes, ce, ve, xl, se, xe);
+      }
+    }
+    if (act) {
+      if (vec) {
+        store2(x + id.row, xe, xo);
+      } else {
+        x[id.row] = xe;
+        if (id.odd) x[id.row + 1] = xo;
+      }
+    }
+  }
+  if (SYM3 && chunks > 1) {
+    // colour 6 backward of a line in chunks, once every colour 7 row is final
+    __syncthreads();
+    for (int t = tid; t < cnt; t += nb) {
+      const PairId id = pair_of(A, C, j0, t, 3);
+      RowVals<VT> ve;
+      T xh[4][4], xl[5][4];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) ve.load(A.vals, id.ke, p, NeedAll());
+#pragma unroll
+      for (int l = 0; l < 9; ++l)
+        load_line(A, id, (const T *)x + id.row, l, true, vec,
+                  l < 4 ? xh[l < 4 ? l : 0] : xl[l < 4 ? 0 : l - 4], 4);
+      const T sum = gs_head<0, false>(holes, ce, ve, xh, vec_to(r[id.row], T()));
+      x[id.row] = gs_tail<0, false>(holes, ce, ve, xl, sum, xl[0][1]);
+    }
   }
 }
 
-// The last class of a forward sweep fused with the first class of the
-// following backward sweep, over the lines [j0, j1) of class 3: colour 6
-// forward, colour 7 forward and backward (SYM), colour 6 backward.  Class 3's
-// colours only depend on each other along x inside a line, so the block's own
-// lines carry every dependency; the matrix rows of the class are read from
-// DRAM once instead of twice (colour 6's rows come back from L2 in the last
-// phase).
-template <int MODE, class VT, class T, class RT>
-__device__ __forceinline__ void gs_lines_sym3(const LevelMat<VT> &A, const ClassInfo &C, int j0,
-                                              int j1, const RT *__restrict__ r, T *x) {
-  constexpr bool ZERO = (MODE & GS_ZERO_GUESS) != 0, STN = (MODE & GS_STENCIL) != 0;
-  const int cnt0 = (j1 - j0) * C.len[0], cnt1 = (j1 - j0) * C.len[1];
-  for (int t = threadIdx.x; t < cnt0; t += blockDim.x)
-    gs_row<ZERO, false, false, false, STN>(A, row_of(C, A.nx, A.ny, 0, j0, t), 6, r, x,
-                                           (const T *)nullptr, (T *)nullptr);
-  __syncthreads();
-  for (int t = threadIdx.x; t < cnt1; t += blockDim.x)
-    gs_row<ZERO, false, false, true, STN>(A, row_of(C, A.nx, A.ny, 1, j0, t), 7, r, x,
-                                          (const T *)nullptr, (T *)nullptr);
-  __syncthreads();
-  // Colour 6 backward multiplies every slot; after a zero-guess forward part,
-  // rows of colours 6 and 7 in other blocks may still be unwritten, which the
-  // exact columns of slots without a neighbour never reach.
-  for (int t = threadIdx.x; t < cnt0; t += blockDim.x)
-    gs_row<false, false, false, false, STN>(A, row_of(C, A.nx, A.ny, 0, j0, t), 6, r, x,
-                                            (const T *)nullptr, (T *)nullptr);
-}
-
-// A half sweep over one class, lpb lines per block.  MODE bits:
-// GS_ZERO_GUESS for the whole launch; GS_PROLONG and GS_RESTRICT act on
-// colour 0 only.  QS >= 0 fixes the class at compile time, which lets the
-// zero-guess sweep drop the loads of the skipped slots statically.
-// Occupancy: the FP64 sweeps stream 12 B per slot and saturate HBM with two
-// 256-thread blocks per SM; the BF16 sweeps read 2 B per slot and are latency
-// bound, so they are held to 64 registers for four blocks per SM (five,
-// at 48 registers, spill and run slower).
-template <class VT>
-constexpr int gs_min_blocks() { return std::is_same<VT, uint16_t>::value ? 4 : 2; }
-
-// Lines [jbeg, jend) of the class, lpb per block (a sharded sweep splits its
-// first launch into the lines that read no halo plane and the rest).
-template <int MODE, int DIR, int QS, class VT, class T, class RT>
-__global__ void __launch_bounds__(kThreads, gs_min_blocks<VT>())
-k_gs_class(LevelMat<VT> A, ClassInfo C, int lpb, int jbeg, int jend, const RT *__restrict__ r,
-           T *x, const T *__restrict__ xc, T *__restrict__ rc, const int *__restrict__ done) {
+// A half sweep over the lines [jbeg, jend) of a class, lpb lines per block (a
+// sharded sweep splits its first launch into the lines that read no halo plane
+// and the rest).  Q >= 0 fixes the class at compile time, which lets the
+// zero-guess sweep drop the loads of the skipped slots.
+// GEN: the general form, for vectors without two-element alignment and matrices
+// with left-out entries; the other form has neither test in it.
+// Against one row per thread with a second load phase for the second colour
+// (before) the pair issues all its loads once: FP64, HBM-bound, the symmetric
+// sweep at 256^3 takes 1186 us = 6.4 TB/s of 8 B per nonzero and pass (before,
+// with stored columns: 1596 us), the V-cycle at 104^3, latency-bound on its
+// coarse levels, 399 us (545).  BF16: 2 B per nonzero leaves the loads' latency
+// and x, which every class launch gathers again, as the bound: V-cycle at
+// 256^3 1137 us (1205), at 64^3 218 us (269).
+template <int MODE, int DIR, int Q, int MINB, bool GEN, class VT, class T, class RT>
+__global__ void __launch_bounds__(kThreads, MINB)
+k_gs_class(LevelMat<VT> A, ClassInfo C, int lpb, int jbeg, int jend, int vec,
+           const RT *__restrict__ r, T *x, const T *__restrict__ xc, T *__restrict__ rc,
+           const int *__restrict__ done) {
+  constexpr bool ZERO = (MODE & GS_ZERO_GUESS) != 0;
+  static_assert(!ZERO || Q >= 0, "the zero-guess sweep knows its class");
+  __shared__ T sh[kThreads + 2];
   if (done && *done) return;
   const int j0 = jbeg + blockIdx.x * lpb;
-  const int j1 = min(j0 + lpb, jend);
-  gs_lines<MODE, QS, DIR>(A, C, j0, j1, r, x, xc, rc);
-}
-
-template <int MODE, class VT, class T, class RT>
-__global__ void __launch_bounds__(kThreads, gs_min_blocks<VT>())
-k_gs_class3_sym(LevelMat<VT> A, ClassInfo C, int lpb, const RT *__restrict__ r, T *x,
-                const int *__restrict__ done) {
-  if (done && *done) return;
-  const int j0 = blockIdx.x * lpb;
-  const int j1 = min(j0 + lpb, C.lines);
-  gs_lines_sym3<MODE>(A, C, j0, j1, r, x);
+  gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0>(
+      A, C, 2 * (Q >= 0 ? Q : C.q), j0, min(j0 + lpb, jend), false, (MODE & GS_PROLONG) != 0,
+      (MODE & GS_RESTRICT) != 0, !GEN || vec, GEN && A.holes, r, x, xc, rc, sh);
 }
 
 // Residual restricted at the injected points (colour 0: even ix, iy, iz):
@@ -738,7 +876,6 @@ __global__ void __launch_bounds__(kThreads)
 k_restrict_residual(LevelMat<VT> A, ClassInfo C0, int64_t nc, const RT *__restrict__ rf,
                     const T *__restrict__ x, T *__restrict__ rc, const int *__restrict__ done) {
   if (done && *done) return;
-  constexpr bool IMPLICIT = std::is_same<VT, uint16_t>::value;
   const int nxc = A.nx >> 1, nyc = A.ny >> 1;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nc;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -754,11 +891,8 @@ k_restrict_residual(LevelMat<VT> A, ClassInfo C0, int64_t nc, const RT *__restri
     int32_t col[HPCGX_STENCIL];
     T val[HPCGX_STENCIL];
 #pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      load_vals(A.vals, id.k, p, NeedAll(), val + 9 * p);
-      if (!IMPLICIT) load_plane(A.cols, id.k, p, NeedAll(), col + 9 * p);
-    }
-    if (IMPLICIT) stencil_cols<true>(A, id, NeedAll(), col);
+    for (int p = 0; p < 3; ++p) load_vals(A.vals, id.k, p, NeedAll(), val + 9 * p);
+    stencil_cols(A, id, val, col);
     check_cols(A, col, NeedAll(), 7);
     T ax = T(0);
 #pragma unroll
@@ -996,6 +1130,7 @@ __global__ void k_copy_z(int64_t n, const double *__restrict__ r, double *z,
 struct Geo {
   int nx, ny, nz;
   int zlo, zhi;   // z-slab: the planes below / above belong to a neighbouring rank
+  int holes;      // the matrix leaves out entries of existing neighbours
   int64_t cstart[8], ccount[8];
   int len[2];
   int nyq[4];
@@ -1042,23 +1177,18 @@ __device__ __forceinline__ bool neighbour(const Geo &g, int ix, int iy, int iz, 
 
 // The reference problem (src/GenerateProblem_ref.cpp:152-172) written
 // straight into the device layout: 26 on the diagonal, -1 elsewhere.
-__global__ void k_generate_hpcg(Geo g, int64_t storage_rows, double *vals, int32_t *cols) {
+__global__ void k_generate_hpcg(Geo g, int64_t storage_rows, double *vals) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < storage_rows;
        k += (int64_t)gridDim.x * blockDim.x) {
     int64_t row;
     int ix, iy, iz;
     const bool real = storage_to_natural(g, k, row, ix, iy, iz);
     for (int s = 0; s < HPCGX_STENCIL; ++s) {
-      int64_t col = 0;
+      int64_t col;
       double v = 0.0;
-      if (real) {
-        if (neighbour(g, ix, iy, iz, s, row, col))
-          v = (s == HPCGX_DIAG_SLOT) ? 26.0 : -1.0;
-        else
-          col = row;
-      }
+      if (real && neighbour(g, ix, iy, iz, s, row, col))
+        v = (s == HPCGX_DIAG_SLOT) ? 26.0 : -1.0;
       vals[vidx(k, s)] = v;
-      cols[cidx(k, s)] = (int32_t)col;
     }
   }
 }
@@ -1067,7 +1197,7 @@ __global__ void k_generate_hpcg(Geo g, int64_t storage_rows, double *vals, int32
 // undirected edge {lo, hi} draws z ~ N(0,1) keyed by the finest-level index of
 // lo and the direction, a = -exp(sigma z); diagonal = sum |a| + 2.
 __global__ void k_generate_varcoef(Geo g, int64_t storage_rows, int level, int nx0, int ny0,
-                                   uint64_t seed, double sigma, double *vals, int32_t *cols) {
+                                   uint64_t seed, double sigma, double *vals) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < storage_rows;
        k += (int64_t)gridDim.x * blockDim.x) {
     int64_t row;
@@ -1075,28 +1205,21 @@ __global__ void k_generate_varcoef(Geo g, int64_t storage_rows, int level, int n
     const bool real = storage_to_natural(g, k, row, ix, iy, iz);
     double dsum = 0.0;
     for (int s = 0; s < HPCGX_STENCIL; ++s) {
-      int64_t col = 0;
+      int64_t col;
       double v = 0.0;
-      if (real) {
-        if (neighbour(g, ix, iy, iz, s, row, col)) {
-          if (s != HPCGX_DIAG_SLOT) {
-            int lx = ix, ly = iy, lz = iz, h = s - 14;
-            if (s < HPCGX_DIAG_SLOT) {
-              lx = ix + (s % 3 - 1);
-              ly = iy + ((s / 3) % 3 - 1);
-              lz = iz + (s / 9 - 1);
-              h = 12 - s;
-            }
-            const int64_t lo = ((int64_t)(lz << level) * ny0 + (ly << level)) * nx0 + (lx << level);
-            v = -exp(sigma * normal01(seed, (uint64_t)lo * 13u + (uint64_t)h));
-            dsum += fabs(v);
-          }
-        } else {
-          col = row;
+      if (real && s != HPCGX_DIAG_SLOT && neighbour(g, ix, iy, iz, s, row, col)) {
+        int lx = ix, ly = iy, lz = iz, h = s - 14;
+        if (s < HPCGX_DIAG_SLOT) {
+          lx = ix + (s % 3 - 1);
+          ly = iy + ((s / 3) % 3 - 1);
+          lz = iz + (s / 9 - 1);
+          h = 12 - s;
         }
+        const int64_t lo = ((int64_t)(lz << level) * ny0 + (ly << level)) * nx0 + (lx << level);
+        v = -exp(sigma * normal01(seed, (uint64_t)lo * 13u + (uint64_t)h));
+        dsum += fabs(v);
       }
       vals[vidx(k, s)] = v;
-      cols[cidx(k, s)] = (int32_t)col;
     }
     if (real) vals[vidx(k, HPCGX_DIAG_SLOT)] = dsum + 2.0;
   }
@@ -1160,14 +1283,26 @@ __global__ void k_set_values(Geo g, int64_t n, const double *__restrict__ in, do
   }
 }
 
-__global__ void k_get_values(Geo g, int64_t n, const double *__restrict__ vals,
-                             const int32_t *__restrict__ cols, double *out, int32_t *cout) {
+// The column of (row, s): the neighbour, or the row itself where it has none or
+// the matrix leaves the entry out (holes, value 0).
+__device__ __forceinline__ int64_t column(const Geo &g, int ix, int iy, int iz, int s, int64_t row,
+                                          double v) {
+  int64_t col;
+  const bool has = neighbour(g, ix, iy, iz, s, row, col);
+  return has && !(g.holes && v == 0.0) ? col : row;
+}
+
+__global__ void k_get_values(Geo g, int64_t n, const double *__restrict__ vals, double *out,
+                             int32_t *cout) {
   for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
        row += (int64_t)gridDim.x * blockDim.x) {
     const int64_t k = natural_to_storage(g, row);
+    const int ix = (int)(row % g.nx), iy = (int)((row / g.nx) % g.ny),
+              iz = (int)(row / ((int64_t)g.nx * g.ny));
     for (int s = 0; s < HPCGX_STENCIL; ++s) {
-      if (out) out[row * HPCGX_STENCIL + s] = vals[vidx(k, s)];
-      if (cout) cout[row * HPCGX_STENCIL + s] = cols[cidx(k, s)];
+      const double v = vals[vidx(k, s)];
+      if (out) out[row * HPCGX_STENCIL + s] = v;
+      if (cout) cout[row * HPCGX_STENCIL + s] = (int32_t)column(g, ix, iy, iz, s, row, v);
     }
   }
 }
@@ -1190,7 +1325,7 @@ __global__ void k_get_diagonal(Geo g, int64_t n, const double *__restrict__ vals
 
 // dL/da_ij = -lambda_i x_j for every stored slot, natural row order, 27 slots
 // per row (zero where the stencil has no neighbour).
-__global__ void k_adjoint_grad(Geo g, int64_t n, const int32_t *__restrict__ cols,
+__global__ void k_adjoint_grad(Geo g, int64_t n, const double *__restrict__ vals,
                                const double *__restrict__ lambda, const double *__restrict__ x,
                                double *grad) {
   for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
@@ -1202,7 +1337,8 @@ __global__ void k_adjoint_grad(Geo g, int64_t n, const int32_t *__restrict__ col
     for (int s = 0; s < HPCGX_STENCIL; ++s) {
       int64_t col;
       const bool has = neighbour(g, ix, iy, iz, s, row, col);
-      grad[row * HPCGX_STENCIL + s] = has ? -(li * x[__ldg(cols + cidx(k, s))]) : 0.0;
+      if (has && g.holes) col = column(g, ix, iy, iz, s, row, vals[vidx(k, s)]);
+      grad[row * HPCGX_STENCIL + s] = has ? -(li * x[col]) : 0.0;
     }
   }
 }
@@ -1214,6 +1350,7 @@ Geo geo_of(const LevelDev &L) {
   g.nz = L.nz;
   g.zlo = L.zlo;
   g.zhi = L.zhi;
+  g.holes = L.holes;
   for (int c = 0; c < 8; ++c) {
     g.cstart[c] = L.cstart[c];
     g.ccount[c] = L.ccount[c];
@@ -1233,7 +1370,6 @@ template <class VT>
 LevelMat<VT> mat_of(const LevelDev &L, const VT *vals) {
   LevelMat<VT> A;
   A.vals = vals;
-  A.cols = L.cols;
   for (int s = 0; s < HPCGX_STENCIL; ++s)
     A.off[s] = (s / 9 - 1) * L.nx * L.ny + ((s / 3) % 3 - 1) * L.nx + (s % 3 - 1);
   A.nx = L.nx;
@@ -1245,22 +1381,28 @@ LevelMat<VT> mat_of(const LevelDev &L, const VT *vals) {
   A.lo = L.zlo ? -L.nx * L.ny : 0;
   A.span = (int)L.n - A.lo + (L.zhi ? L.nx * L.ny : 0);
   A.srows = L.storage_rows;
+  A.holes = L.holes;
   return A;
 }
 
-// The SpMV's blocks: `groups` Gauss-Seidel line groups per block (the SpMV has
-// no colour order, so a block can take several and amortise its epilogue,
-// the fused dot product's block reduction).
-ClassSet classes_of(const LevelDev &L, int groups = 1) {
+// Vector loads of x, y and the right-hand side: every line starts on an even
+// row and the vectors on a two-element boundary (a halo plane of an odd size
+// or a view at an odd offset does not).
+template <class T>
+bool aligned2(const T *v) {
+  return reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0;
+}
+
+// The SpMV's blocks: 256 consecutive pairs of a class each.
+ClassSet classes_of(const LevelDev &L) {
   ClassSet cs;
   cs.common = INT_MAX;
   cs.total = 0;
   for (int q = 0; q < 4; ++q) {
     const ClassInfo &C = L.cls[q];
-    const int lpb = std::min(L.lines_per_block[q] * groups, std::max(C.lines, 1));
+    const int64_t pairs = (int64_t)C.lines * C.len[0];
     cs.c[q] = C;
-    cs.lpb[q] = lpb;
-    cs.nblk[q] = C.lines > 0 ? (C.lines + lpb - 1) / lpb : 0;
+    cs.nblk[q] = (int)((pairs + kThreads - 1) / kThreads);
     cs.common = std::min(cs.common, cs.nblk[q]);
     cs.total += cs.nblk[q];
   }
@@ -1307,14 +1449,7 @@ void plan_level(LevelDev &L, int nx, int ny, int nz) {
     C.dlen[0] = make_fastdiv((uint32_t)C.len[0]);
     C.dlen[1] = make_fastdiv((uint32_t)C.len[1]);
     C.dnyq = make_fastdiv((uint32_t)C.nyq);
-    const int len = std::max(C.len[0], 1);
-    int lpb = std::max(1, kThreads / len);
-    lpb = std::min(lpb, std::max(C.lines, 1));
-    L.lines_per_block[q] = lpb;
-    L.blocks[q] = C.lines > 0 ? (C.lines + lpb - 1) / lpb : 0;
-    int th = std::min(kThreads, ((lpb * len) + 31) / 32 * 32);
-    L.threads[q] = std::max(th, 32);
-    L.spmv_blocks += L.blocks[q];
+    L.spmv_blocks += (int)(((int64_t)C.lines * C.len[0] + kThreads - 1) / kThreads);
   }
 }
 
@@ -1327,15 +1462,14 @@ int64_t storage_row_host(const LevelDev &L, int64_t row) {
 }
 
 int launch_generate_hpcg(const LevelDev &L, cudaStream_t s) {
-  k_generate_hpcg<<<grid_for(L.storage_rows), kThreads, 0, s>>>(geo_of(L), L.storage_rows, L.vals,
-                                                                L.cols);
+  k_generate_hpcg<<<grid_for(L.storage_rows), kThreads, 0, s>>>(geo_of(L), L.storage_rows, L.vals);
   return 1;
 }
 
 int launch_generate_varcoef(const LevelDev &L, int level, int nx0, int ny0, uint64_t seed,
                             double sigma, cudaStream_t s) {
   k_generate_varcoef<<<grid_for(L.storage_rows), kThreads, 0, s>>>(
-      geo_of(L), L.storage_rows, level, nx0, ny0, seed, sigma, L.vals, L.cols);
+      geo_of(L), L.storage_rows, level, nx0, ny0, seed, sigma, L.vals);
   return 1;
 }
 
@@ -1357,7 +1491,7 @@ int launch_set_values(const LevelDev &L, const double *vals27, cudaStream_t s) {
 }
 
 int launch_get_values(const LevelDev &L, double *vals27, int32_t *cols27, cudaStream_t s) {
-  k_get_values<<<grid_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, L.cols, vals27, cols27);
+  k_get_values<<<grid_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, vals27, cols27);
   return 1;
 }
 
@@ -1372,35 +1506,31 @@ int launch_get_diagonal(const LevelDev &L, double *diag, cudaStream_t s) {
 }
 
 int launch_spmv(const LevelDev &L, const double *x, double *y, const Reduce *dot, int fin,
-                void *fin_target, const int *done, cudaStream_t s, bool implicit_cols) {
+                void *fin_target, const int *done, cudaStream_t s) {
   if (L.spmv_blocks == 0) return 0;
-  implicit_cols = implicit_cols || L.stencil_cols;
-  // measured at 512^3: two line groups per block help the stencil-column
-  // SpMV (4.77 against 5.11 ms with the fused dot product), not the other
-  const ClassSet cs = classes_of(L, implicit_cols ? 2 : 1);
+  const ClassSet cs = classes_of(L);
   const LevelMat<double> A = mat_of(L, L.vals);
+  const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(y);
   const Reduce red = dot ? *dot : Reduce();
-  if (dot && implicit_cols)
-    k_spmv<double, double, true, true><<<cs.total, kThreads, 0, s>>>(A, cs, x, y, red, fin,
-                                                                     fin_target, done);
-  else if (dot)
-    k_spmv<double, double, true, false><<<cs.total, kThreads, 0, s>>>(A, cs, x, y, red, fin,
-                                                                      fin_target, done);
-  else if (implicit_cols)
-    k_spmv<double, double, false, true><<<cs.total, kThreads, 0, s>>>(A, cs, x, y, red, 0,
-                                                                      nullptr, done);
-  else
-    k_spmv<double, double, false, false><<<cs.total, kThreads, 0, s>>>(A, cs, x, y, red, 0,
-                                                                       nullptr, done);
-  return 1;
+  auto go = [&](auto kernel) {
+    kernel<<<cs.total, kThreads, 0, s>>>(A, cs, x, y, vec, red, fin, fin_target, done);
+    return 1;
+  };
+  if (vec && !L.holes)
+    return dot ? go(k_spmv<double, double, true, false>) : go(k_spmv<double, double, false, false>);
+  return dot ? go(k_spmv<double, double, true, true>) : go(k_spmv<double, double, false, true>);
 }
 
 int launch_spmv32(const LevelDev &L, const float *x, float *y, cudaStream_t s) {
   if (L.spmv_blocks == 0) return 0;
-  const ClassSet cs = classes_of(L, 2);
-  k_spmv<uint16_t, float, false, true><<<cs.total, kThreads, 0, s>>>(
-      mat_of(L, L.vals16), cs, x, y, Reduce(), 0, nullptr, nullptr);
-  return 1;
+  const ClassSet cs = classes_of(L);
+  const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(y);
+  auto go = [&](auto kernel) {
+    kernel<<<cs.total, kThreads, 0, s>>>(mat_of(L, L.vals16), cs, x, y, vec, Reduce(), 0, nullptr,
+                                         nullptr);
+    return 1;
+  };
+  return vec ? go(k_spmv<uint16_t, float, false, false>) : go(k_spmv<uint16_t, float, false, true>);
 }
 
 template <class T>
@@ -1416,60 +1546,82 @@ struct ValsOf<float> {
   static const uint16_t *get(const LevelDev &L) { return L.vals16; }
 };
 
-// The class kernels.  EXTRA: GS_STENCIL (FP64: columns from the stencil
-// offsets), added to every launch's mode.
-template <int EXTRA, class T, class RT>
+// The block of a class launch: whole lines.  FP64: a pair needs some 220
+// registers, so two blocks of 128 threads share an SM and one loads while the
+// other computes (V-cycle at 256^3: 2490 us against 2623 with blocks of 256; 128
+// registers for two blocks of 256 spill: 4061).  BF16: blocks of up to 256.  A
+// class of few lines takes fewer lines per block so that there is a block for
+// each SM twice over (a launch is then bound by one block's latency).
+struct GsBlock {
+  int lines, threads;
+};
+template <class T>
+GsBlock gs_block(const ClassInfo &C) {
+  const int target = std::is_same<T, double>::value ? 128 : kThreads;
+  const int len = C.len[0];
+  const int lines = std::min(std::max(1, target / len), std::max(1, C.lines / (2 * 148)));
+  return {lines, std::min(kThreads, (lines * len + 31) / 32 * 32)};
+}
+
+// Pairs of a class from which the BF16 sweeps give up registers (105 -> 80, a
+// few spilled) for a third block per SM: with several waves of blocks another
+// block hides a block's latency (V-cycle at 384^3 3292 us against 3814), with
+// about one wave it does not come to run (64^3: 218 against 228 us).
+constexpr int64_t kManyPairs = 100000;
+
+// The class kernels, by blocks per SM and form (k_gs_class).
+template <int MINB, bool GEN, class T, class RT>
 int launch_gs_rows(const LevelDev &L, int q, int backward, int mode, const RT *r, T *x,
-                   const T *xc, T *rc, const int *done, cudaStream_t s, int jbeg, int jend) {
+                   const T *xc, T *rc, const int *done, cudaStream_t s, int jbeg, int jend,
+                   GsBlock gb, int vec) {
   using VT = typename ValsOf<T>::VT;
-  const LevelMat<VT> A = mat_of(L, ValsOf<T>::get(L));
-  const int lpb = L.lines_per_block[q];
-  const dim3 g((unsigned)((jend - jbeg + lpb - 1) / lpb)), b(L.threads[q]);
+  LevelMat<VT> A = mat_of(L, ValsOf<T>::get(L));
+  // left-out entries are a matter of the FP64 operators; the BF16 copy
+  // multiplies the neighbour by 0
+  if (!std::is_same<T, double>::value) A.holes = 0;
+  const dim3 g((unsigned)((jend - jbeg + gb.lines - 1) / gb.lines)), b(gb.threads);
   const ClassInfo &C = L.cls[q];
-  if (mode & GS_SYM3) {
-    if (q != 3) return 0;
-    if (mode & GS_ZERO_GUESS)
-      k_gs_class3_sym<GS_ZERO_GUESS | EXTRA><<<g, b, 0, s>>>(A, C, lpb, r, x, done);
-    else
-      k_gs_class3_sym<GS_PLAIN | EXTRA><<<g, b, 0, s>>>(A, C, lpb, r, x, done);
+  auto go = [&](auto kernel) {
+    kernel<<<g, b, 0, s>>>(A, C, gb.lines, jbeg, jend, vec, r, x, xc, rc, done);
     return 1;
-  }
+  };
+  if (mode == GS_SYM3 && q == 3) return go(k_gs_class<GS_SYM3, 0, 3, MINB, GEN, VT, T, RT>);
+  if (mode == (GS_SYM3 | GS_ZERO_GUESS) && q == 3)
+    return go(k_gs_class<GS_SYM3 | GS_ZERO_GUESS, 0, 3, MINB, GEN, VT, T, RT>);
   if (mode == GS_ZERO_GUESS && !backward) {
     switch (q) {
-      case 0: k_gs_class<GS_ZERO_GUESS | EXTRA, 0, 0><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done); break;
-      case 1: k_gs_class<GS_ZERO_GUESS | EXTRA, 0, 1><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done); break;
-      case 2: k_gs_class<GS_ZERO_GUESS | EXTRA, 0, 2><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done); break;
-      default: k_gs_class<GS_ZERO_GUESS | EXTRA, 0, 3><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done); break;
+      case 0: return go(k_gs_class<GS_ZERO_GUESS, 0, 0, MINB, GEN, VT, T, RT>);
+      case 1: return go(k_gs_class<GS_ZERO_GUESS, 0, 1, MINB, GEN, VT, T, RT>);
+      case 2: return go(k_gs_class<GS_ZERO_GUESS, 0, 2, MINB, GEN, VT, T, RT>);
+      default: return go(k_gs_class<GS_ZERO_GUESS, 0, 3, MINB, GEN, VT, T, RT>);
     }
-    return 1;
   }
-  if (mode == GS_RESTRICT && backward && q == 0) {
-    k_gs_class<GS_RESTRICT | EXTRA, 1, 0><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done);
-    return 1;
-  }
-  if (mode == GS_PROLONG && !backward && q == 0) {
-    k_gs_class<GS_PROLONG | EXTRA, 0, 0><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done);
-    return 1;
-  }
+  if (mode == GS_RESTRICT && backward && q == 0)
+    return go(k_gs_class<GS_RESTRICT, 1, 0, MINB, GEN, VT, T, RT>);
+  if (mode == GS_PROLONG && !backward && q == 0)
+    return go(k_gs_class<GS_PROLONG, 0, 0, MINB, GEN, VT, T, RT>);
   if (mode != GS_PLAIN) return 0;
-  if (backward)
-    k_gs_class<GS_PLAIN | EXTRA, 1, -1><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done);
-  else
-    k_gs_class<GS_PLAIN | EXTRA, 0, -1><<<g, b, 0, s>>>(A, C, lpb, jbeg, jend, r, x, xc, rc, done);
-  return 1;
+  return backward ? go(k_gs_class<GS_PLAIN, 1, -1, MINB, GEN, VT, T, RT>)
+                  : go(k_gs_class<GS_PLAIN, 0, -1, MINB, GEN, VT, T, RT>);
 }
 
 template <class T, class RT>
 int launch_gs_class(const LevelDev &L, int q, int backward, int mode, const RT *r, T *x,
                     const T *xc, T *rc, const int *done, cudaStream_t s, int jbeg, int jend) {
   if (jend < 0) jend = L.cls[q].lines;
-  if (L.blocks[q] == 0 || jend <= jbeg) return 0;
+  if (jend <= jbeg) return 0;
   if ((mode & GS_SYM3) && (jbeg != 0 || jend != L.cls[q].lines)) return 0;   // whole class only
-  if constexpr (std::is_same<T, double>::value) {
-    if (L.stencil_cols)
-      return launch_gs_rows<GS_STENCIL>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg, jend);
-  }
-  return launch_gs_rows<0>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg, jend);
+  const GsBlock gb = gs_block<T>(L.cls[q]);
+  const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(r);
+  constexpr bool fp64 = std::is_same<T, double>::value;
+  if (!vec || (fp64 && L.holes))
+    return launch_gs_rows<fp64 ? 1 : 2, true>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg,
+                                              jend, gb, vec);
+  if (!fp64 && (int64_t)L.cls[q].lines * L.cls[q].len[0] > kManyPairs)
+    return launch_gs_rows<fp64 ? 1 : 3, false>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg,
+                                               jend, gb, vec);
+  return launch_gs_rows<fp64 ? 1 : 2, false>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg,
+                                             jend, gb, vec);
 }
 
 template <class T, class RT>
@@ -1639,7 +1791,7 @@ int launch_copy_z(int64_t n, const double *r, double *z, const CgState *st, cuda
 
 int launch_adjoint_grad(const LevelDev &L, const double *lambda, const double *x, double *grad,
                         cudaStream_t s) {
-  k_adjoint_grad<<<grid_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.cols, lambda, x, grad);
+  k_adjoint_grad<<<grid_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, lambda, x, grad);
   return 1;
 }
 

@@ -13,17 +13,14 @@ struct LevelDev {
   int64_t storage_rows = 0;   // rows incl. the padding that aligns colours to 32
   int64_t cstart[8] = {}, ccount[8] = {};
   ClassInfo cls[4] = {};
-  int lines_per_block[4] = {}, blocks[4] = {}, threads[4] = {};
-  int spmv_blocks = 0;        // all four classes in one launch (one line group per block)
-  // FP64 operators derive their columns from the stencil offsets instead of
-  // reading the int32 column arrays (hpcgx_set_stencil_columns)
-  bool stencil_cols = false;
+  int spmv_blocks = 0;        // all four classes in one launch
+  // a loaded matrix that leaves out entries of existing neighbours (LevelMat)
+  bool holes = false;
   // z-slab of a sharded problem: a neighbouring rank owns the plane below
   // (zlo) / above (zhi); vectors read by SpMV and Gauss-Seidel then hold one
   // halo plane on each side (indices -nx*ny..-1 and n..n+nx*ny-1)
   int zlo = 0, zhi = 0;
   double *vals = nullptr;     // storage_rows*27, FP64
-  int32_t *cols = nullptr;    // storage_rows*27
   uint16_t *vals16 = nullptr; // storage_rows*27, BF16 (mixed precision)
   // multigrid work vectors of this level (levels >= 1: right-hand side and
   // correction; level 0 uses the caller's vectors)
@@ -72,10 +69,7 @@ enum GsMode : int {
   GS_ZERO_GUESS = 1,
   GS_RESTRICT = 2,
   GS_PROLONG = 4,
-  GS_SYM3 = 8,
-  // internal to the kernels: the FP64 sweeps derive their columns from the
-  // stencil offsets (LevelDev::stencil_cols)
-  GS_STENCIL = 32
+  GS_SYM3 = 8
 };
 
 // Layout / set-up ---------------------------------------------------------
@@ -92,9 +86,8 @@ int launch_set_diagonal(const LevelDev &L, const double *diag, cudaStream_t s);
 int launch_get_diagonal(const LevelDev &L, double *diag, cudaStream_t s);
 
 // Operators ---------------------------------------------------------------
-// implicit_cols: columns from the stencil offsets (no int32 column reads).
 int launch_spmv(const LevelDev &L, const double *x, double *y, const Reduce *dot, int fin,
-                 void *fin_target, const int *done, cudaStream_t s, bool implicit_cols = false);
+                 void *fin_target, const int *done, cudaStream_t s);
 int launch_spmv32(const LevelDev &L, const float *x, float *y, cudaStream_t s);
 // One class launch of a Gauss-Seidel half sweep over lines [jbeg, jend) of
 // the class (default: all).  T = double (FP64 values and vectors) or float

@@ -127,7 +127,7 @@ int set_error(int code, const char *msg) { return fail(code, msg); }
 }  // namespace hpcgx
 
 // 32-row slices per chunk of the host loaders' pinned staging (2 chunks of
-// 4096 x 864 values and columns: 2 x 42 MB)
+// 4096 x 864 values: 2 x 28 MB)
 constexpr int64_t kPinnedSlices = 4096;
 
 static int env_int(const char *name, int dflt) {
@@ -209,16 +209,14 @@ struct hpcgx_problem {
     return HPCGX_OK;
   }
   // ---- pinned host staging of the host loaders: two chunks of kPinnedSlices
-  // 32-row slices (values and columns), allocated on the first load
+  // 32-row slices of values, allocated on the first load
   double *pin_vals[2] = {};
-  int32_t *pin_cols[2] = {};
   cudaEvent_t pin_copied[2] = {};
   int pinned_staging() {
     if (pin_vals[0]) return HPCGX_OK;
     const size_t e = (size_t)kPinnedSlices * kSliceElems;
     for (int h = 0; h < 2; ++h) {
       CK(cudaHostAlloc((void **)&pin_vals[h], e * sizeof(double), cudaHostAllocDefault));
-      CK(cudaHostAlloc((void **)&pin_cols[h], e * sizeof(int32_t), cudaHostAllocDefault));
       CK(cudaEventCreateWithFlags(&pin_copied[h], cudaEventDisableTiming));
     }
     return HPCGX_OK;
@@ -254,9 +252,7 @@ struct hpcgx_problem {
   // ---- byte model of one class launch (for probes)
   double gs_bytes(int l, int q, int mode, bool mixed, double rb0 = 8.0) const {
     const LevelDev &A = L[l];
-    // mixed: BF16 value per slot, columns derived from the stencil offsets
-    // (FP64 with stencil columns: no column reads either)
-    const double vb = mixed ? 2.0 : 8.0, cb = (mixed || A.stencil_cols) ? 0.0 : 4.0;
+    const double vb = mixed ? 2.0 : 8.0;   // the value of a slot; no column is stored
     const double xb = mixed ? 4.0 : 8.0;
     const double rb = l > 0 ? (mixed ? 4.0 : 8.0) : rb0;
     double total = 0.0;
@@ -268,9 +264,7 @@ struct hpcgx_problem {
         const int dx = s % 3 - 1, dy = (s / 3) % 3 - 1, dz = s / 9 - 1;
         const int64_t cnt = axis_count(A.nx, px, dx) * axis_count(A.ny, py, dy) *
                             axis_count(A.nz, pz, dz);
-        const bool skipped = (mode == GS_ZERO_GUESS) && s != HPCGX_DIAG_SLOT &&
-                             ((c ^ slot_mask(s)) > c);
-        nnzb += (double)cnt * (skipped ? vb : vb + cb);
+        nnzb += (double)cnt * vb;
       }
       double vec = rows * (rb + xb + ((mode & GS_ZERO_GUESS) ? 0.0 : xb));
       // (GS_SYM3: the class's matrix, right-hand side and x once; the second
@@ -448,13 +442,9 @@ struct hpcgx_problem {
       vec_bytes(16.0 + 24.0 + 16.0);
     }
     if (capturing) CK(cudaEventRecordWithFlags(phase[kind][2], stream, cudaEventRecordExternal));
-    // The mixed solver's FP64 SpMV derives its columns from the stencil
-    // offsets; the plain FP64 solver reads the int32 column arrays.
-    const bool implicit_cols = kind == G_MIXED || L[0].stencil_cols;
     double spmv_bytes = 0.0;
     if ((probe & HPCGX_PROBE_SPMV_FINE) || capturing) {
-      // 12 B (8 B without column reads) per real nonzero, x and y once; the
-      // fused p.Ap reads nothing extra
+      // 8 B per real nonzero, x and y once; the fused p.Ap reads nothing extra
       int64_t nnz = 0;
       for (int s = 0; s < HPCGX_STENCIL; ++s) {
         const int dx = s % 3 - 1, dy = (s / 3) % 3 - 1, dz = s / 9 - 1;
@@ -464,10 +454,10 @@ struct hpcgx_problem {
         for (int i = 0; i < L[0].nz; ++i) cz += (i + dz >= 0 && i + dz < L[0].nz);
         nnz += cx * cy * cz;
       }
-      spmv_bytes = (implicit_cols ? 8.0 : 12.0) * nnz + 16.0 * n;
+      spmv_bytes = 8.0 * nnz + 16.0 * n;
     }
     TRY(probed(HPCGX_PROBE_SPMV_FINE, spmv_bytes, [&]() {
-      return launch_spmv(L[0], p, Ap, &red, FIN_CG_PAP, st, done, stream, implicit_cols);
+      return launch_spmv(L[0], p, Ap, &red, FIN_CG_PAP, st, done, stream);
     }));
     if (capturing) CK(cudaEventRecordWithFlags(phase[kind][3], stream, cudaEventRecordExternal));
     float *r32_out = (kind == G_MIXED && fine_r32) ? r32 : nullptr;
@@ -551,7 +541,7 @@ struct hpcgx_problem {
     // that the iteration graph never changes
     if (xu != x) CK(cudaMemcpyAsync(x, xu, n * sizeof(double), cudaMemcpyDeviceToDevice, stream));
     CK(cudaMemcpyAsync(p, x, n * sizeof(double), cudaMemcpyDeviceToDevice, stream));
-    note(launch_spmv(L[0], p, Ap, nullptr, 0, nullptr, nullptr, stream, kind == G_MIXED));
+    note(launch_spmv(L[0], p, Ap, nullptr, 0, nullptr, nullptr, stream));
     note(launch_cg_init(n, bu, Ap, r, (kind == G_MIXED && fine_r32) ? r32 : nullptr, red, st,
                         stream));
     TRY(build_graph(kind));
@@ -796,7 +786,7 @@ struct hpcgx_problem {
     return HPCGX_OK;
   }
   // CG set-up (src/CG.cpp:86-92): p = x, Ap = A p, r = b - Ap, normr0.
-  void plan_cg_init(Plan &pl, int kind, const double *bu) {
+  void plan_cg_init(Plan &pl, const double *bu) {
     const int64_t n = L[0].n;
     add(pl, [=]() {
       CK(cudaMemcpyAsync(p, x, n * sizeof(double), cudaMemcpyDeviceToDevice, stream));
@@ -804,7 +794,7 @@ struct hpcgx_problem {
     });
     add_halo(pl, 0, p, sizeof(double));
     add(pl, [=]() {
-      note(launch_spmv(L[0], p, Ap, nullptr, 0, nullptr, nullptr, stream, kind == G_MIXED));
+      note(launch_spmv(L[0], p, Ap, nullptr, 0, nullptr, nullptr, stream));
       return HPCGX_OK;
     });
     add(pl, [=]() {
@@ -846,7 +836,7 @@ struct hpcgx_problem {
     add_halo(pl, 0, p, sizeof(double));
     add(pl, [=]() {
       const Reduce d = deferred();
-      note(launch_spmv(L[0], p, Ap, &d, FIN_CG_PAP, st, done, stream, mixed));
+      note(launch_spmv(L[0], p, Ap, &d, FIN_CG_PAP, st, done, stream));
       return HPCGX_OK;
     });
     add_sum(pl, FIN_CG_PAP, 1);
@@ -879,7 +869,6 @@ hpcgx_problem::~hpcgx_problem() {
   }
   for (int l = 0; l < kMaxLevels; ++l) {
     cudaFree(L[l].vals);
-    cudaFree(L[l].cols);
     cudaFree(L[l].vals16);
     cudaFree(L[l].r64);
     cudaFree(L[l].r32);
@@ -889,7 +878,6 @@ hpcgx_problem::~hpcgx_problem() {
   for (int h = 0; h < 2; ++h) {
     if (pin_copied[h]) cudaEventDestroy(pin_copied[h]);
     if (pin_vals[h]) cudaFreeHost(pin_vals[h]);
-    if (pin_cols[h]) cudaFreeHost(pin_cols[h]);
   }
   for (void *ptr : {(void *)b, (void *)x, (void *)r, (void *)r32, (void *)Ap, (void *)tmp,
                     (void *)result,
@@ -977,7 +965,7 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
   auto scan_row = [&](int64_t row, auto put) -> std::string {
     const int ix = (int)(row % A.nx), iy = (int)((row / A.nx) % A.ny),
               iz = (int)(row / ((int64_t)A.nx * A.ny));
-    for (int s = 0; s < HPCGX_STENCIL; ++s) put(s, (int32_t)row, 0.0);
+    for (int s = 0; s < HPCGX_STENCIL; ++s) put(s, 0.0);
     const int nz = nnz_of(row);
     if (nz < 1 || nz > HPCGX_STENCIL) return std::to_string(nz) + " entries";
     int last = -1;
@@ -996,7 +984,7 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
       if (s <= last) return "entries not in stencil order";
       last = s;
       diag |= (s == HPCGX_DIAG_SLOT);
-      put(s, col, v);
+      put(s, v);
     }
     if (!diag) return "no diagonal";
     return std::string();
@@ -1008,8 +996,9 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
   int64_t off[HPCGX_STENCIL];
   for (int s = 0; s < HPCGX_STENCIL; ++s)
     off[s] = (s % 3 - 1) + (int64_t)A.nx * ((s / 3) % 3 - 1 + (int64_t)A.ny * (s / 9 - 1));
+  std::atomic<bool> holes{false};
   auto fast_row = [&](int64_t row, int ix, int iy, int iz, auto put) -> bool {
-    for (int s = 0; s < HPCGX_STENCIL; ++s) put(s, (int32_t)row, 0.0);
+    for (int s = 0; s < HPCGX_STENCIL; ++s) put(s, 0.0);
     const int nz = nnz_of(row);
     if (nz < 1 || nz > HPCGX_STENCIL) return false;
     const bool okx[3] = {ix > 0, true, ix + 1 < A.nx}, oky[3] = {iy > 0, true, iy + 1 < A.ny},
@@ -1025,9 +1014,12 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
         if (okx[s % 3] && oky[(s / 3) % 3] && okz[s / 9] && row + off[s] == col) break;
       }
       diag |= (s == HPCGX_DIAG_SLOT);
-      put(s, col, v);
+      put(s, v);
       ++s;
     }
+    // an existing neighbour without an entry
+    if (nz < (okx[0] + 1 + okx[2]) * (oky[0] + 1 + oky[2]) * (okz[0] + 1 + okz[2]))
+      holes.store(true, std::memory_order_relaxed);
     return diag;
   };
   p->loaded[level] = false;
@@ -1040,7 +1032,6 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
   for (int64_t c0 = 0, it = 0; c0 < slices && !failed; c0 += kPinnedSlices, ++it) {
     const int h = (int)(it & 1);
     double *bv = p->pin_vals[h];
-    int32_t *bc = p->pin_cols[h];
     if (pending[h]) CK(cudaEventSynchronize(p->pin_copied[h]));
     pending[h] = false;
     const int64_t c1 = std::min(slices, c0 + kPinnedSlices);
@@ -1049,17 +1040,11 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
       for (int64_t k = k0 + a; k < k0 + e; ++k) {
         int ix, iy, iz;
         const int64_t row = natural_row_host(A, k, ix, iy, iz);
-        if (row < 0) {   // padding: value 0, column 0
-          for (int s = 0; s < HPCGX_STENCIL; ++s) {
-            bv[vidx(k, s) - e0] = 0.0;
-            bc[cidx(k, s) - e0] = 0;
-          }
+        if (row < 0) {   // padding
+          for (int s = 0; s < HPCGX_STENCIL; ++s) bv[vidx(k, s) - e0] = 0.0;
           continue;
         }
-        auto put = [&](int s, int32_t col, double v) {
-          bv[vidx(k, s) - e0] = v;
-          bc[cidx(k, s) - e0] = col;
-        };
+        auto put = [&](int s, double v) { bv[vidx(k, s) - e0] = v; };
         if (!fast_row(row, ix, iy, iz, put) && !scan_row(row, put).empty()) {
           bad[t] = 1;
           return;
@@ -1070,8 +1055,6 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
     if (failed) break;
     const size_t ne = (size_t)(c1 - c0) * kSliceElems;
     CK(cudaMemcpyAsync(A.vals + e0, bv, ne * sizeof(double), cudaMemcpyHostToDevice, p->stream));
-    CK(cudaMemcpyAsync(A.cols + e0, bc, ne * sizeof(int32_t), cudaMemcpyHostToDevice,
-                       p->stream));
     CK(cudaEventRecord(p->pin_copied[h], p->stream));
     pending[h] = true;
   }
@@ -1082,7 +1065,7 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
     std::vector<std::string> msg(64);
     parallel_for(A.n, [&](int64_t a, int64_t e, int t) {
       for (int64_t row = a; row < e; ++row) {
-        const std::string m = scan_row(row, [](int, int32_t, double) {});
+        const std::string m = scan_row(row, [](int, double) {});
         if (!m.empty()) {
           first[t] = row;
           msg[t] = m;
@@ -1094,6 +1077,7 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
       if (first[t] >= 0) return fail(HPCGX_ELAYOUT, "row " + std::to_string(first[t]) + ": " + msg[t]);
     return fail(HPCGX_ELAYOUT, "malformed row");
   }
+  A.holes = holes.load();
   p->loaded[level] = true;
   return HPCGX_OK;
 }
@@ -1434,7 +1418,7 @@ int sharded_cg(const std::vector<hpcgx_problem *> &ps, const Runner &run, int ki
     CK(cudaMemcpyAsync(p->st, &h, sizeof(h), cudaMemcpyHostToDevice, p->stream));
     CK(cudaMemcpyAsync(p->x, x[r], p->L[0].n * sizeof(double), cudaMemcpyDeviceToDevice,
                        p->stream));
-    p->plan_cg_init(init[r], kind, b[r]);
+    p->plan_cg_init(init[r], b[r]);
     p->plan_cg_iteration(iter[r], kind);
   }
   TRY(run(init));
@@ -1547,7 +1531,6 @@ int hpcgx_create_slab(int device, int nx, int ny, int nz, int levels, int nranks
     A.zhi = rank + 1 < nranks;
     const size_t slots = (size_t)A.storage_rows * HPCGX_STENCIL;
     if ((rc = p->alloc((void **)&A.vals, slots * sizeof(double)))) return bail(rc);
-    if ((rc = p->alloc((void **)&A.cols, slots * sizeof(int32_t)))) return bail(rc);
     const int64_t plane = (int64_t)A.nx * A.ny;
     if (l > 0) {
       if ((rc = p->alloc((void **)&A.r64, A.n * sizeof(double)))) return bail(rc);
@@ -1556,8 +1539,6 @@ int hpcgx_create_slab(int device, int nx, int ny, int nz, int levels, int nranks
       if ((rc = p->alloc_halo((void **)&A.x32, A.n, sizeof(float), plane))) return bail(rc);
     }
     red_cap = std::max<int64_t>(red_cap, red_need(A.spmv_blocks));
-    for (int q = 0; q < 4; ++q)
-      red_cap = std::max<int64_t>(red_cap, red_need(A.blocks[q]));
   }
   const int64_t n = p->L[0].n;
   red_cap = std::max<int64_t>(red_cap, red_need(vector_blocks(n)));
@@ -1713,6 +1694,7 @@ int hpcgx_generate(hpcgx_problem *p, int kind, uint64_t seed, double sigma) {
     } else {
       return fail(HPCGX_EINVAL, "unknown generator kind");
     }
+    p->L[l].holes = false;
     p->loaded[l] = true;
   }
   CK(cudaStreamSynchronize(p->stream));
@@ -1733,16 +1715,8 @@ int hpcgx_build_mixed(hpcgx_problem *p) {
 
 int hpcgx_set_stencil_columns(hpcgx_problem *p, int on) {
   HANDLE(p);
-  TRY(stencil_only(p, "hpcgx_set_stencil_columns"));
-  for (int l = 0; l < p->nlev; ++l) p->L[l].stencil_cols = on != 0;
-  // the FP64 iteration graphs hold the other kernels: rebuild them on next use
-  for (int k : {G_FP64_PREC, G_FP64_NOPREC})
-    if (p->graph[k]) {
-      CK(cudaGraphExecDestroy(p->graph[k]));
-      p->graph[k] = nullptr;
-      p->probes[k].clear();
-    }
-  return HPCGX_OK;
+  (void)on;   // every operator derives its columns; nothing to switch
+  return stencil_only(p, "hpcgx_set_stencil_columns");
 }
 
 int hpcgx_set_diagonal_host(hpcgx_problem *p, int level, const double *diag) {
@@ -1782,10 +1756,12 @@ int hpcgx_set_values(hpcgx_problem *p, int level, const double *vals27, int reco
   TRY(stencil_only(p, "hpcgx_set_values"));
   TRY(check_level(p, level));
   p->note(launch_set_values(p->L[level], vals27, p->stream));
+  p->L[level].holes = false;
   p->loaded[level] = true;
   if (recoarsen)
     for (int l = level; l + 1 < p->nlev; ++l) {
       p->note(launch_coarsen_varcoef(p->L[l], p->L[l + 1], p->stream));
+      p->L[l + 1].holes = false;
       p->loaded[l + 1] = true;
     }
   CK(cudaStreamSynchronize(p->stream));
@@ -1838,7 +1814,7 @@ int hpcgx_spmv_stencil(hpcgx_problem *p, int level, const double *x, double *y) 
   if (p->nranks > 1) return fail(HPCGX_ESTATE, "not available on a sharded problem");
   TRY(check_level(p, level));
   if (!p->loaded[level]) return fail(HPCGX_ESTATE, "level not loaded");
-  p->note(launch_spmv(p->L[level], x, y, nullptr, 0, nullptr, nullptr, p->stream, true));
+  p->note(launch_spmv(p->L[level], x, y, nullptr, 0, nullptr, nullptr, p->stream));
   CK(cudaStreamSynchronize(p->stream));
   CK(cudaGetLastError());
   return HPCGX_OK;

@@ -281,8 +281,8 @@ class Problem:
         check(lib().hpcgx_build_mixed(self.h))
 
     def set_stencil_columns(self, on=True):
-        """FP64 operators derive their columns from the stencil offsets (the
-        mixed solver always does); same results, no int32 column reads."""
+        """Every operator derives its columns from the stencil offsets whatever
+        ``on`` says; kept for callers that asked for it."""
         check(lib().hpcgx_set_stencil_columns(self.h, int(bool(on))))
 
     def set_diagonal(self, level, diag):
@@ -321,7 +321,7 @@ class Problem:
         return _dev(t, self.rows(level), dtypes, self.device, name)
 
     def spmv(self, x, level=0, y=None, stencil_cols=False):
-        """y = A x; stencil_cols derives the columns from the stencil offsets."""
+        """y = A x (stencil_cols: hpcgx_spmv_stencil, the same product)."""
         self._pre()
         y = self.empty(level) if y is None else y
         f = lib().hpcgx_spmv_stencil if stencil_cols else lib().hpcgx_spmv

@@ -103,12 +103,10 @@ int hpcgx_check_f2c(hpcgx_problem *p, int level, const int32_t *f2c_host, int64_
 int hpcgx_generate(hpcgx_problem *p, int kind, uint64_t seed, double sigma);
 /* Builds (or refreshes) the BF16 value copies used by the mixed solver. */
 int hpcgx_build_mixed(hpcgx_problem *p);
-/* on != 0: the FP64 operators (SpMV, SYMGS, MG, CG) derive every column from
- * the level's stencil offsets instead of reading the int32 column arrays, as
- * the mixed solver always does (no reference counterpart; loaded levels are
- * 27-point stencil matrices, so the results are the same bits).  This is the
- * FP64 solve to compare the mixed one with when only the precision differs.
- * Default off. */
+/* Kept for callers of the FP64 operators that asked for derived columns: every
+ * operator derives its columns from the level's stencil offsets now (loaded
+ * levels are 27-point stencil matrices, so no column is stored), whatever `on`
+ * says.  HPCGX_ESTATE on a general-pattern problem. */
 int hpcgx_set_stencil_columns(hpcgx_problem *p, int on);
 /* Coherence with ReplaceMatrixDiagonal (src/SparseMatrix.hpp:139-145):
  * writes level `level`'s diagonal from host memory. */
@@ -129,10 +127,8 @@ int64_t hpcgx_rows(hpcgx_problem *p, int level);
 
 /* ComputeSPMV (src/ComputeSPMV.hpp:20): y = A_level x. */
 int hpcgx_spmv(hpcgx_problem *p, int level, const double *x, double *y);
-/* y = A_level x in FP64 with every column derived from the stencil offsets
- * (row + offset) instead of read from the int32 column arrays: the outer SpMV
- * of the mixed solver (no reference counterpart).  Loaded matrices are
- * 27-point stencil matrices, so the sums are those of hpcgx_spmv. */
+/* The product of hpcgx_spmv, which derives its columns too; refused on a
+ * sharded or a general-pattern problem. */
 int hpcgx_spmv_stencil(hpcgx_problem *p, int level, const double *x, double *y);
 /* ComputeSYMGS (src/ComputeSYMGS.hpp:20): one symmetric Gauss-Seidel sweep in
  * colour order (forward colours 0..7, backward 7..0), x updated in place. */
