@@ -145,6 +145,36 @@ __device__ __forceinline__ double mac_sub(double s, double a, double b) {
 __device__ __forceinline__ float mac_add(float s, float a, float b) { return __fmaf_rn(a, b, s); }
 __device__ __forceinline__ float mac_sub(float s, float a, float b) { return __fmaf_rn(-a, b, s); }
 
+// Programmatic dependent launch: a kernel launched by launch_dependent starts
+// while the kernel before it on the stream still runs, and reads or writes
+// nothing that a kernel may have produced or may still read until
+// dependency_wait returns; all it may do before is index arithmetic and loads
+// of matrix values.  dependents_launch lets the kernel after it start in the
+// same way, once every block of this one has called it.  A kernel that returns
+// early waits first, or the one after it would not wait for the one before it.
+// Pointers to data of other kernels are not __restrict__ const in such a
+// kernel, nor read with __ldg: such loads count as invariant and may be moved
+// ahead of the wait.
+__device__ __forceinline__ void dependents_launch() {
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Matrix value -> arithmetic type.
 __device__ __forceinline__ double to_arith(double v, double) { return v; }
 __device__ __forceinline__ float to_arith(uint16_t h, float) {

@@ -585,24 +585,35 @@ __device__ __forceinline__ T term_sub(bool holes, T sum, T v, T x) {
 // (128 registers, two blocks per SM); one and three blocks measured the same.
 template <class VT, class T, bool DOT, bool GEN>
 __global__ void __launch_bounds__(kThreads, std::is_same<VT, double>::value ? 2 : 4)
-k_spmv(LevelMat<VT> A, ClassSet cs, const T *__restrict__ x, T *__restrict__ y, int wide,
-       Reduce red, int fin, void *fin_target, const int *__restrict__ done) {
-  if (done && *done) return;
+k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet cs, const T *x,
+       T *y, int wide, Reduce red, int fin, void *fin_target, const int *done) {
+  dependents_launch();
   const bool vec = !GEN || wide, holes = GEN && A.holes;
   int q, b;
   class_block(cs, (int)blockIdx.x, q, b);
   const ClassInfo &C = cs.c[q];
   const int t = b * kThreads + (int)threadIdx.x;
   double acc = 0.0;
-  if (t < C.lines * C.len[0]) {
-    const PairId id = pair_of(A, C, 0, t, 1);
+  const bool act = t < C.lines * C.len[0];
+  PairId id;
+  T ve[9], vo[9];
+  if (act) {
+    id = pair_of(A, C, 0, t, 1);
+    load_vals(A.vals, id.ke, 0, NeedAll(), ve);
+    load_vals(A.vals, id.ko, 0, NeedAll(), vo);
+  }
+  dependency_wait();
+  if (done && *done) return;
+  if (act) {
     const T *xr = x + id.row;
     T se = T(0), so = T(0), xe = T(0), xo = T(0);
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-      T ve[9], vo[9], v[3][4];
-      load_vals(A.vals, id.ke, p, NeedAll(), ve);
-      load_vals(A.vals, id.ko, p, NeedAll(), vo);
+      T v[3][4];
+      if (p > 0) {
+        load_vals(A.vals, id.ke, p, NeedAll(), ve);
+        load_vals(A.vals, id.ko, p, NeedAll(), vo);
+      }
 #pragma unroll
       for (int i = 0; i < 3; ++i) load_line(A, id, xr, 3 * p + i, true, vec, v[i], 2);
 #pragma unroll
@@ -696,14 +707,17 @@ __device__ __forceinline__ T gs_tail(bool holes, int c, const V &val, const T (&
 //       halo holds the slab below's smoothed values).
 // SYM3: forward and backward half sweep of the last class (DIR = 0): colour 6
 //       forward, colour 7 forward and backward, colour 6 backward.
+// AHEAD: the matrix values are loaded before the kernel ahead is waited for
+// (launch_dependent); done: nothing to do once it is set.
 // Lines longer than a block are taken in chunks of blockDim pairs, from right
 // to left forward and from left to right backward: a chunk then finds the
 // neighbours that its first row must see unchanged unchanged, and those that
 // its second row must see updated updated.
-template <int DIR, bool ZERO, bool SYM3, class VT, class T, class RT>
+template <int DIR, bool ZERO, bool SYM3, bool AHEAD, class VT, class T, class RT>
 __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo &C, int ce, int j0,
                                          int j1, bool zero, bool pro, bool res, bool vec,
-                                         bool holes, const RT *r, T *x, const T *xc, T *rc, T *sh) {
+                                         bool holes, const RT *r, T *x, const T *xc, T *rc, T *sh,
+                                         const int *done) {
   const int cnt = (j1 - j0) * C.len[0];
   const int nb = blockDim.x, tid = threadIdx.x;
   const int chunks = (cnt + nb - 1) / nb;
@@ -720,8 +734,23 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
     T xl[5][4];
     T se = T(0), so = T(0), ax = T(0), xe = T(0), xo = T(0), re = T(0);
     int64_t crow = 0;
+    if (!AHEAD && ch == 0) {
+      dependency_wait();
+      if (done && *done) return;
+    }
     if (act) {
       id = pair_of(A, C, j0, t, 3);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        ve.load(A.vals, id.ke, p, need_e);
+        vo.load(A.vals, id.ko, p, need_o);
+      }
+    }
+    if (AHEAD && ch == 0) {
+      dependency_wait();
+      if (done && *done) return;
+    }
+    if (act) {
       const T *xr = x + id.row;
       T ro = T(0);
       if (vec) {
@@ -735,11 +764,6 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
       }
       {
         T xh[4][4];
-#pragma unroll
-        for (int p = 0; p < 3; ++p) {
-          ve.load(A.vals, id.ke, p, need_e);
-          vo.load(A.vals, id.ko, p, need_o);
-        }
 #pragma unroll
         for (int l = 0; l < 9; ++l) {
           T *to = l < 4 ? xh[l < 4 ? l : 0] : xl[l < 4 ? 0 : l - 4];
@@ -849,19 +873,24 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
 // coarse levels, 399 us (545).  BF16: 2 B per nonzero leaves the loads' latency
 // and x, which every class launch gathers again, as the bound: V-cycle at
 // 256^3 1137 us (1205), at 64^3 218 us (269).
+// Launched dependent on the launch before (launch_dependent): the launch, the
+// index arithmetic and the values' loads go under the end of that one, 49
+// times in a V-cycle: FP64 at 104^3 279 us (399), at 256^3 2341 us (2513);
+// BF16 at 64^3 136 us (218), at 256^3 937 us (1137), at 384^3 2934 us (3293).
+// The BF16 kernels with three blocks per SM wait first (AHEAD off): values held
+// over the wait cost them spills (384^3: 3353 us).
 template <int MODE, int DIR, int Q, int MINB, bool GEN, class VT, class T, class RT>
 __global__ void __launch_bounds__(kThreads, MINB)
-k_gs_class(LevelMat<VT> A, ClassInfo C, int lpb, int jbeg, int jend, int vec,
-           const RT *__restrict__ r, T *x, const T *__restrict__ xc, T *__restrict__ rc,
-           const int *__restrict__ done) {
+k_gs_class(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassInfo C, int lpb,
+           int jbeg, int jend, int vec, const RT *r, T *x, const T *xc, T *rc, const int *done) {
   constexpr bool ZERO = (MODE & GS_ZERO_GUESS) != 0;
   static_assert(!ZERO || Q >= 0, "the zero-guess sweep knows its class");
   __shared__ T sh[kThreads + 2];
-  if (done && *done) return;
+  dependents_launch();
   const int j0 = jbeg + blockIdx.x * lpb;
-  gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0>(
+  gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0, MINB != 3>(
       A, C, 2 * (Q >= 0 ? Q : C.q), j0, min(j0 + lpb, jend), false, (MODE & GS_PROLONG) != 0,
-      (MODE & GS_RESTRICT) != 0, !GEN || vec, GEN && A.holes, r, x, xc, rc, sh);
+      (MODE & GS_RESTRICT) != 0, !GEN || vec, GEN && A.holes, r, x, xc, rc, sh, done);
 }
 
 // Residual restricted at the injected points (colour 0: even ix, iy, iz):
@@ -1038,8 +1067,9 @@ k_cg_init(int64_t n, const double *__restrict__ b, const double *__restrict__ Ap
 // rtz = r.z (src/CG.cpp:109/112); for the flexible solver also z.Ap_{k-1}.
 template <class ZT, bool FLEX>
 __global__ void __launch_bounds__(kThreads)
-k_cg_rz(int64_t n, const double *__restrict__ r, const ZT *__restrict__ z,
-        const double *__restrict__ Ap, Reduce red, CgState *st) {
+k_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, Reduce red, CgState *st) {
+  dependents_launch();
+  dependency_wait();
   if (st->done) return;
   const bool two = FLEX && st->k > 1;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1067,8 +1097,9 @@ k_cg_rz(int64_t n, const double *__restrict__ r, const ZT *__restrict__ z,
 // k_cg_xflush applies the last iteration's update after the loop.
 template <class ZT>
 __global__ void __launch_bounds__(kThreads)
-k_cg_p(int64_t n, const ZT *__restrict__ z, double *p, const CgState *__restrict__ st,
-       double *x) {
+k_cg_p(int64_t n, const ZT *z, double *p, const CgState *st, double *x) {
+  dependents_launch();
+  dependency_wait();
   if (st->done) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const bool first = st->k == 1;
@@ -1099,8 +1130,10 @@ k_cg_xflush(int64_t n, const double *__restrict__ p, double *x, const CgState *_
 // (src/CG.cpp:121-124).  r32 (mixed solver): the FP32 copy of r that the
 // V-cycle's finest level reads -- the value it would round r to itself.
 __global__ void __launch_bounds__(kThreads)
-k_cg_xr(int64_t n, const double *__restrict__ p, const double *__restrict__ Ap, double *x,
-        double *r, float *r32, Reduce red, CgState *st) {
+k_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32,
+        Reduce red, CgState *st) {
+  dependents_launch();
+  dependency_wait();
   if (st->done) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const double alpha = st->alpha, malpha = -st->alpha;
@@ -1513,7 +1546,8 @@ int launch_spmv(const LevelDev &L, const double *x, double *y, const Reduce *dot
   const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(y);
   const Reduce red = dot ? *dot : Reduce();
   auto go = [&](auto kernel) {
-    kernel<<<cs.total, kThreads, 0, s>>>(A, cs, x, y, vec, red, fin, fin_target, done);
+    launch_dependent(kernel, dim3(cs.total), dim3(kThreads), s, A, cs, x, y, vec, red, fin,
+                     fin_target, done);
     return 1;
   };
   if (vec && !L.holes)
@@ -1526,8 +1560,8 @@ int launch_spmv32(const LevelDev &L, const float *x, float *y, cudaStream_t s) {
   const ClassSet cs = classes_of(L);
   const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(y);
   auto go = [&](auto kernel) {
-    kernel<<<cs.total, kThreads, 0, s>>>(mat_of(L, L.vals16), cs, x, y, vec, Reduce(), 0, nullptr,
-                                         nullptr);
+    launch_dependent(kernel, dim3(cs.total), dim3(kThreads), s, mat_of(L, L.vals16), cs, x, y, vec,
+                     Reduce(), 0, (void *)nullptr, (const int *)nullptr);
     return 1;
   };
   return vec ? go(k_spmv<uint16_t, float, false, false>) : go(k_spmv<uint16_t, float, false, true>);
@@ -1582,7 +1616,7 @@ int launch_gs_rows(const LevelDev &L, int q, int backward, int mode, const RT *r
   const dim3 g((unsigned)((jend - jbeg + gb.lines - 1) / gb.lines)), b(gb.threads);
   const ClassInfo &C = L.cls[q];
   auto go = [&](auto kernel) {
-    kernel<<<g, b, 0, s>>>(A, C, gb.lines, jbeg, jend, vec, r, x, xc, rc, done);
+    launch_dependent(kernel, g, b, s, A, C, gb.lines, jbeg, jend, vec, r, x, xc, rc, done);
     return 1;
   };
   if (mode == GS_SYM3 && q == 3) return go(k_gs_class<GS_SYM3, 0, 3, MINB, GEN, VT, T, RT>);
@@ -1753,9 +1787,9 @@ template <class ZT>
 int launch_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, const Reduce &red,
                  CgState *st, cudaStream_t s) {
   if (Ap)
-    k_cg_rz<ZT, true><<<vector_blocks(n), kThreads, 0, s>>>(n, r, z, Ap, red, st);
+    launch_dependent(k_cg_rz<ZT, true>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap, red, st);
   else
-    k_cg_rz<ZT, false><<<vector_blocks(n), kThreads, 0, s>>>(n, r, z, Ap, red, st);
+    launch_dependent(k_cg_rz<ZT, false>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap, red, st);
   return 1;
 }
 template int launch_cg_rz<double>(int64_t, const double *, const double *, const double *,
@@ -1765,7 +1799,7 @@ template int launch_cg_rz<float>(int64_t, const double *, const float *, const d
 
 template <class ZT>
 int launch_cg_p(int64_t n, const ZT *z, double *p, CgState *st, cudaStream_t s, double *x) {
-  k_cg_p<ZT><<<vector_blocks(n), kThreads, 0, s>>>(n, z, p, st, x);
+  launch_dependent(k_cg_p<ZT>, dim3(vector_blocks(n)), dim3(kThreads), s, n, z, p, st, x);
   return 1;
 }
 template int launch_cg_p<double>(int64_t, const double *, double *, CgState *, cudaStream_t,
@@ -1780,7 +1814,7 @@ int launch_cg_xflush(int64_t n, const double *p, double *x, const CgState *st, c
 
 int launch_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32,
                  const Reduce &red, CgState *st, cudaStream_t s) {
-  k_cg_xr<<<vector_blocks(n), kThreads, 0, s>>>(n, p, Ap, x, r, r32, red, st);
+  launch_dependent(k_cg_xr, dim3(vector_blocks(n)), dim3(kThreads), s, n, p, Ap, x, r, r32, red, st);
   return 1;
 }
 

@@ -402,6 +402,9 @@ struct hpcgx_problem {
         if (!A.vals16) TRY(alloc((void **)&A.vals16, A.storage_rows * HPCGX_STENCIL * 2));
         note(launch_to_bf16(A, stream));
       }
+      // the sweeps load matrix values before they wait for the kernel ahead of
+      // them (launch_dependent)
+      CK(cudaStreamSynchronize(stream));
       mixed_ready = true;
       mixed_stale = false;
     }
