@@ -166,12 +166,15 @@ struct GeneralProblem {
   int64_t launches = 0;
   // CG
   double *r = nullptr, *z = nullptr, *p = nullptr, *Ap = nullptr;
+  double *x = nullptr;             // the solution vector of the graphs
   CgState *st = nullptr;
   Reduce red;
-  cudaGraphExec_t graph[2] = {};
-  const double *graph_x[2] = {};   // the solution vector a graph was captured for
+  // one iteration without and with preconditioner, without [0] and with [1] the
+  // events that time its phases
+  cudaGraphExec_t graph[2][2] = {};
   cudaEvent_t phase[2][5] = {};
-  bool capturing = false;
+  bool timed = false;              // capturing with events
+  CgMonitor monitor;
 
   int alloc(void **ptr, size_t n) {
     cudaError_t e = cudaMalloc(ptr, std::max<size_t>(n, 8));
@@ -186,7 +189,8 @@ struct GeneralProblem {
   }
   ~GeneralProblem() {
     for (int k = 0; k < 2; ++k) {
-      if (graph[k]) cudaGraphExecDestroy(graph[k]);
+      for (cudaGraphExec_t exec : graph[k])
+        if (exec) cudaGraphExecDestroy(exec);
       for (cudaEvent_t &ev : phase[k])
         if (ev) cudaEventDestroy(ev);
     }
@@ -235,20 +239,20 @@ struct GeneralProblem {
   void iteration(int precond, double *x) {
     const int64_t n = L[0].n;
     const int *done = &st->done;
-    if (capturing) cudaEventRecordWithFlags(phase[precond][0], stream, cudaEventRecordExternal);
+    if (timed) cudaEventRecordWithFlags(phase[precond][0], stream, cudaEventRecordExternal);
     if (precond)
       mg(0, r, z, done);
     else
       note(launch_copy_z(n, r, z, st, stream));
-    if (capturing) cudaEventRecordWithFlags(phase[precond][1], stream, cudaEventRecordExternal);
+    if (timed) cudaEventRecordWithFlags(phase[precond][1], stream, cudaEventRecordExternal);
     note(launch_cg_rz<double>(n, r, z, nullptr, red, st, stream));
     note(launch_cg_p<double>(n, z, p, st, stream));
-    if (capturing) cudaEventRecordWithFlags(phase[precond][2], stream, cudaEventRecordExternal);
+    if (timed) cudaEventRecordWithFlags(phase[precond][2], stream, cudaEventRecordExternal);
     spmv(0, p, Ap, done);
     note(launch_dot_finish(n, p, Ap, red, FIN_CG_PAP, st, stream));
-    if (capturing) cudaEventRecordWithFlags(phase[precond][3], stream, cudaEventRecordExternal);
+    if (timed) cudaEventRecordWithFlags(phase[precond][3], stream, cudaEventRecordExternal);
     note(launch_cg_xr(n, p, Ap, x, r, nullptr, red, st, stream));
-    if (capturing) cudaEventRecordWithFlags(phase[precond][4], stream, cudaEventRecordExternal);
+    if (timed) cudaEventRecordWithFlags(phase[precond][4], stream, cudaEventRecordExternal);
   }
 };
 
@@ -276,11 +280,12 @@ GeneralProblem *general_create(int nlev, cudaStream_t s) {
 void general_destroy(GeneralProblem *g) { delete g; }
 void general_set_stream(GeneralProblem *g, cudaStream_t s) {
   g->stream = s;
-  for (int k = 0; k < 2; ++k)
-    if (g->graph[k]) {
-      cudaGraphExecDestroy(g->graph[k]);
-      g->graph[k] = nullptr;
-    }
+  for (auto &kind : g->graph)
+    for (cudaGraphExec_t &exec : kind)
+      if (exec) {
+        cudaGraphExecDestroy(exec);
+        exec = nullptr;
+      }
 }
 
 int64_t general_rows(const GeneralProblem *g, int level) {
@@ -463,7 +468,7 @@ int general_load_level(GeneralProblem *g, int level, int64_t n, const char *nnz,
   GCK(cudaMemcpyAsync(A.diag, hdiag.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
   if (coarse) GCK(cudaMemcpyAsync(A.f2c, f2c, nc * sizeof(int32_t), cudaMemcpyHostToDevice, s));
   if (level == 0) {
-    for (double **v : {&g->r, &g->z, &g->p, &g->Ap}) GTRY(g->alloc((void **)v, n * sizeof(double)));
+    for (double **v : {&g->r, &g->z, &g->p, &g->Ap, &g->x}) GTRY(g->alloc((void **)v, n * sizeof(double)));
     GTRY(g->alloc((void **)&g->st, sizeof(CgState)));
     const int64_t blocks = vector_blocks(n);
     const int64_t cap = 2 * blocks + 2 * ((blocks + 1023) / 1024);
@@ -510,36 +515,43 @@ int general_cg(GeneralProblem *g, const double *b, double *x, int max_iter, doub
   std::memset(&h, 0, sizeof(h));
   h.tol = tol;
   h.max_iter = max_iter;
+  GCK(g->monitor.init());
+  h.mirror = g->monitor.slots;
   GCK(cudaMemcpyAsync(g->st, &h, sizeof(h), cudaMemcpyHostToDevice, s));
   // p = x, Ap = A p, r = b - Ap, normr0 (src/CG.cpp:86-96)
+  GCK(cudaMemcpyAsync(g->x, x, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   GCK(cudaMemcpyAsync(g->p, x, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   g->spmv(0, g->p, g->Ap, nullptr);
   g->note(launch_cg_init(n, b, g->Ap, g->r, nullptr, g->red, g->st, s));
-  // one CUDA graph per iteration, captured on first use for this x
-  if (!g->graph[kind] || g->graph_x[kind] != x) {
-    if (g->graph[kind]) {
-      GCK(cudaGraphExecDestroy(g->graph[kind]));
-      g->graph[kind] = nullptr;
-    }
-    for (cudaEvent_t &ev : g->phase[kind])
-      if (!ev) GCK(cudaEventCreate(&ev));
+  // one CUDA graph per iteration, captured on first use
+  const bool timed = times != nullptr;
+  cudaGraphExec_t &exec = g->graph[kind][timed];
+  if (!exec) {
+    if (timed)
+      for (cudaEvent_t &ev : g->phase[kind])
+        if (!ev) GCK(cudaEventCreate(&ev));
     cudaGraph_t gr = nullptr;
     GCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    g->capturing = true;
+    g->timed = timed;
     const int64_t before = g->launches;
-    g->iteration(kind, x);
-    g->capturing = false;
+    g->iteration(kind, g->x);
+    g->timed = false;
     g->launches = before;
     GCK(cudaStreamEndCapture(s, &gr));
-    const cudaError_t e = cudaGraphInstantiate(&g->graph[kind], gr, 0);
+    const cudaError_t e = cudaGraphInstantiate(&exec, gr, 0);
     cudaGraphDestroy(gr);
     GCK(e);
-    g->graph_x[kind] = x;
   }
   double t_mg = 0, t_vec = 0, t_spmv = 0;
   int launched = 0;
-  while (launched < max_iter) {
-    GCK(cudaGraphLaunch(g->graph[kind], s));
+  if (!timed) {
+    GCK(g->monitor.run(s, max_iter, &h, [&]() {
+      ++launched;
+      return cudaGraphLaunch(exec, s);
+    }));
+  }
+  while (timed && launched < max_iter) {
+    GCK(cudaGraphLaunch(exec, s));
     ++launched;
     GCK(cudaMemcpyAsync(&h, g->st, sizeof(h), cudaMemcpyDeviceToHost, s));
     GCK(cudaStreamSynchronize(s));
@@ -555,10 +567,10 @@ int general_cg(GeneralProblem *g, const double *b, double *x, int max_iter, doub
     }
     if (h.done) break;
   }
-  if (launched == 0) {
+  if (launched == 0)
     GCK(cudaMemcpyAsync(&h, g->st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    GCK(cudaStreamSynchronize(s));
-  }
+  GCK(cudaMemcpyAsync(x, g->x, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  GCK(cudaStreamSynchronize(s));
   if (niters) *niters = h.niters;
   if (normr) *normr = h.normr;
   if (normr0) *normr0 = h.normr0;

@@ -168,6 +168,8 @@ __device__ void finish(int fin, void *target, const double (&tot)[NV]) {
       st->niters = 0;
       st->nonfinite = !isfinite(st->normr);
       st->done = !(st->normr / st->normr0 > st->tol) || st->max_iter < 1 || st->nonfinite;
+      // a solve that is done here has no iteration that would leave its state
+      if (st->mirror) st->mirror[0] = st->mirror[1] = *st;
       break;
     case FIN_CG_RZ:
       if (st->k == 1) {
@@ -193,6 +195,7 @@ __device__ void finish(int fin, void *target, const double (&tot)[NV]) {
       st->k += 1;
       st->nonfinite = !isfinite(st->normr);
       st->done = !(st->normr / st->normr0 > st->tol) || st->k > st->max_iter || st->nonfinite;
+      if (st->mirror) st->mirror[st->niters & 1] = *st;
       break;
     default:
       break;
@@ -1446,6 +1449,22 @@ ClassSet classes_of(const LevelDev &L) {
 
 // ======================================================================== host
 // Every launch_* returns the number of kernels it launched (0 or 1).
+
+cudaError_t CgMonitor::init() {
+  if (slots) return cudaSuccess;
+  for (cudaEvent_t &e : ev) {
+    const cudaError_t rc = e ? cudaSuccess : cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    if (rc != cudaSuccess) return rc;
+  }
+  const cudaError_t rc = cudaHostAlloc((void **)&slots, 2 * sizeof(CgState), cudaHostAllocMapped);
+  if (rc != cudaSuccess) slots = nullptr;
+  return rc;
+}
+CgMonitor::~CgMonitor() {
+  for (cudaEvent_t e : ev)
+    if (e) cudaEventDestroy(e);
+  if (slots) cudaFreeHost(slots);
+}
 
 int vector_blocks(int64_t n) {
   int64_t b = (n + kThreads * 4 - 1) / (kThreads * 4);

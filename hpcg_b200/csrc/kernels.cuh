@@ -38,6 +38,39 @@ struct CgState {
   int niters;
   int flexible;  // Polak-Ribiere beta for a variable (mixed) preconditioner
   int nonfinite; // a non-finite residual norm stopped the loop
+  // two slots of host memory or null: iteration k leaves this state in slot k & 1
+  CgState *mirror;
+};
+
+// How the host follows a solve without a copy and a wait between iterations:
+// the iteration's last kernel writes the state into pinned memory, and while
+// the host waits for iteration k iteration k + 1 is queued already (its kernels
+// return at once where k was the last).
+struct CgMonitor {
+  CgState *slots = nullptr;      // pinned, device-visible
+  cudaEvent_t ev[2] = {};
+  cudaError_t init();            // on first use
+  ~CgMonitor();
+  // Launches iterations through launch() until one is done or max_iter ran;
+  // *last: the state after the last one.
+  template <class F>
+  cudaError_t run(cudaStream_t s, int max_iter, CgState *last, F launch) {
+    int launched = 0, seen = 0;
+    while (seen < max_iter) {
+      while (launched < max_iter && launched < seen + 2) {
+        ++launched;
+        cudaError_t e = launch();
+        if (e == cudaSuccess) e = cudaEventRecord(ev[launched & 1], s);
+        if (e != cudaSuccess) return e;
+      }
+      ++seen;
+      const cudaError_t e = cudaEventSynchronize(ev[seen & 1]);
+      if (e != cudaSuccess) return e;
+      *last = slots[seen & 1];
+      if (last->done) break;
+    }
+    return cudaSuccess;
+  }
 };
 
 // Scratch of the deterministic grid reductions: per-block partial sums and a

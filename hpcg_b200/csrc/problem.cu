@@ -160,16 +160,18 @@ struct hpcgx_problem {
   double *result = nullptr;   // device scalars of standalone reductions
   CgState *st = nullptr;
   Reduce red;
-  // graphs of one CG iteration
-  cudaGraphExec_t graph[G_COUNT] = {};
+  // graphs of one CG iteration: without [0] and with [1] the events that time
+  // its phases and probed launches
+  cudaGraphExec_t graph[G_COUNT][2] = {};
   int graph_kernels[G_COUNT] = {};
   int graph_probe[G_COUNT] = {};
+  CgMonitor monitor;
   // algorithmic bytes of one iteration of each graph (this implementation's
   // byte model, summed over its launches while the graph is captured)
   double graph_bytes[G_COUNT] = {};
   cudaEvent_t phase[G_COUNT][5] = {};
   // capture bookkeeping
-  bool capturing = false;
+  bool capturing = false, capture_timed = false;
   int capture_kind = 0;
   int64_t launches = 0;
   // probe
@@ -282,7 +284,7 @@ struct hpcgx_problem {
   template <class F>
   int probed(int kinds, double bytes_model, F &&launch) {
     if (capturing) graph_bytes[capture_kind] += bytes_model;
-    const int armed = capturing ? (kinds & probe) : 0;
+    const int armed = capture_timed ? (kinds & probe) : 0;
     if (armed) {
       if (pool_next >= event_pool.size()) return fail(HPCGX_ESTATE, "probe event pool exhausted");
       Probe pr = event_pool[pool_next++];
@@ -424,7 +426,7 @@ struct hpcgx_problem {
     } else {
       TRY((vcycle<float, double>(r, z32, done)));
     }
-    if (capturing) CK(cudaEventRecordWithFlags(phase[kind][1], stream, cudaEventRecordExternal));
+    if (capture_timed) CK(cudaEventRecordWithFlags(phase[kind][1], stream, cudaEventRecordExternal));
     // vector kernels, bytes per row: r.z reads r, z (and Ap); p = z + beta p
     // reads z and p and writes p, and applies the previous iteration's
     // x += alpha p (reads and writes x); r -= alpha Ap reads Ap and reads and
@@ -444,7 +446,7 @@ struct hpcgx_problem {
       note(launch_cg_p<double>(n, z, p, st, stream, x));
       vec_bytes(16.0 + 24.0 + 16.0);
     }
-    if (capturing) CK(cudaEventRecordWithFlags(phase[kind][2], stream, cudaEventRecordExternal));
+    if (capture_timed) CK(cudaEventRecordWithFlags(phase[kind][2], stream, cudaEventRecordExternal));
     double spmv_bytes = 0.0;
     if ((probe & HPCGX_PROBE_SPMV_FINE) || capturing) {
       // 8 B per real nonzero, x and y once; the fused p.Ap reads nothing extra
@@ -462,34 +464,37 @@ struct hpcgx_problem {
     TRY(probed(HPCGX_PROBE_SPMV_FINE, spmv_bytes, [&]() {
       return launch_spmv(L[0], p, Ap, &red, FIN_CG_PAP, st, done, stream);
     }));
-    if (capturing) CK(cudaEventRecordWithFlags(phase[kind][3], stream, cudaEventRecordExternal));
+    if (capture_timed) CK(cudaEventRecordWithFlags(phase[kind][3], stream, cudaEventRecordExternal));
     float *r32_out = (kind == G_MIXED && fine_r32) ? r32 : nullptr;
     note(launch_cg_xr(n, p, Ap, nullptr, r, r32_out, red, st, stream));
     vec_bytes(r32_out ? 28.0 : 24.0);
-    if (capturing) CK(cudaEventRecordWithFlags(phase[kind][4], stream, cudaEventRecordExternal));
+    if (capture_timed) CK(cudaEventRecordWithFlags(phase[kind][4], stream, cudaEventRecordExternal));
     return HPCGX_OK;
   }
 
-  int build_graph(int kind) {
-    if (graph[kind] && graph_probe[kind] == probe) return HPCGX_OK;
-    if (graph[kind]) {
-      cudaGraphExecDestroy(graph[kind]);
-      graph[kind] = nullptr;
-      probes[kind].clear();
+  int build_graph(int kind, bool timed) {
+    cudaGraphExec_t &exec = graph[kind][timed];
+    if (exec && (!timed || graph_probe[kind] == probe)) return HPCGX_OK;
+    if (exec) {
+      cudaGraphExecDestroy(exec);
+      exec = nullptr;
     }
-    for (int i = 0; i < 5; ++i)
-      if (!phase[kind][i]) CK(cudaEventCreate(&phase[kind][i]));
-    // every launch a probe can bracket in one iteration: 14 class launches
-    // per level (two symmetric sweeps of 7), plus the SpMV, with room to spare
-    const size_t need = 16 * kMaxLevels + 1;
-    if (probe != HPCGX_PROBE_NONE) {
-      // events of earlier graphs may still be referenced: keep them, add new
-      while (event_pool.size() - pool_next < need) {
-        Probe pr;
-        CK(cudaEventCreate(&pr.a));
-        CK(cudaEventCreate(&pr.b));
-        pr.bytes = 0.0;
-        event_pool.push_back(pr);
+    if (timed) {
+      probes[kind].clear();
+      for (int i = 0; i < 5; ++i)
+        if (!phase[kind][i]) CK(cudaEventCreate(&phase[kind][i]));
+      // every launch a probe can bracket in one iteration: 14 class launches
+      // per level (two symmetric sweeps of 7), plus the SpMV, with room to spare
+      const size_t need = 16 * kMaxLevels + 1;
+      if (probe != HPCGX_PROBE_NONE) {
+        // events of earlier graphs may still be referenced: keep them, add new
+        while (event_pool.size() - pool_next < need) {
+          Probe pr;
+          CK(cudaEventCreate(&pr.a));
+          CK(cudaEventCreate(&pr.b));
+          pr.bytes = 0.0;
+          event_pool.push_back(pr);
+        }
       }
     }
     cudaGraph_t g = nullptr;
@@ -497,10 +502,11 @@ struct hpcgx_problem {
     graph_bytes[kind] = 0.0;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     capturing = true;
+    capture_timed = timed;
     capture_kind = kind;
-    cudaEventRecordWithFlags(phase[kind][0], stream, cudaEventRecordExternal);
+    if (timed) cudaEventRecordWithFlags(phase[kind][0], stream, cudaEventRecordExternal);
     int rc = iteration(kind);
-    capturing = false;
+    capturing = capture_timed = false;
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     graph_kernels[kind] = (int)(launches - before);
     launches = before;
@@ -509,10 +515,10 @@ struct hpcgx_problem {
       return rc;
     }
     CK(e);
-    e = cudaGraphInstantiate(&graph[kind], g, 0);
+    e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     CK(e);
-    graph_probe[kind] = probe;
+    if (timed) graph_probe[kind] = probe;
     return HPCGX_OK;
   }
 
@@ -539,6 +545,8 @@ struct hpcgx_problem {
     h.tol = tol;
     h.max_iter = max_iter;
     h.flexible = kind == G_MIXED;
+    CK(monitor.init());
+    h.mirror = monitor.slots;
     CK(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, stream));
     // p = x (CopyVector, src/CG.cpp:86); x lives in the problem's own buffer so
     // that the iteration graph never changes
@@ -547,36 +555,49 @@ struct hpcgx_problem {
     note(launch_spmv(L[0], p, Ap, nullptr, 0, nullptr, nullptr, stream));
     note(launch_cg_init(n, bu, Ap, r, (kind == G_MIXED && fine_r32) ? r32 : nullptr, red, st,
                         stream));
-    TRY(build_graph(kind));
-    const bool per_iter = tol > 0.0 || probe != HPCGX_PROBE_NONE || times != nullptr;
+    const bool timed = probe != HPCGX_PROBE_NONE || times != nullptr;
+    TRY(build_graph(kind, timed));
+    const cudaGraphExec_t exec = graph[kind][timed];
     double t_mg = 0, t_vec = 0, t_spmv = 0;
     int launched = 0;
-    while (launched < max_iter) {
-      const int batch = per_iter ? 1 : max_iter - launched;
-      for (int i = 0; i < batch; ++i) {
-        CK(cudaGraphLaunch(graph[kind], stream));
+    if (timed) {
+      // one iteration at a time: the next one records the same events
+      while (launched < max_iter) {
+        CK(cudaGraphLaunch(exec, stream));
+        launches += graph_kernels[kind];
+        ++launched;
+        CK(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, stream));
+        CK(cudaStreamSynchronize(stream));
+        if (h.niters == launched) {
+          float a = 0, b2 = 0, c = 0;
+          CK(cudaEventElapsedTime(&a, phase[kind][0], phase[kind][1]));
+          CK(cudaEventElapsedTime(&b2, phase[kind][1], phase[kind][2]));
+          CK(cudaEventElapsedTime(&c, phase[kind][2], phase[kind][3]));
+          float d = 0;
+          CK(cudaEventElapsedTime(&d, phase[kind][3], phase[kind][4]));
+          t_mg += a * 1e-3;
+          t_vec += (b2 + d) * 1e-3;
+          t_spmv += c * 1e-3;
+          TRY(read_probes(kind));
+        }
+        if (h.done) break;
+      }
+    } else if (tol > 0.0) {
+      CK(monitor.run(stream, max_iter, &h, [&]() {
+        ++launched;
+        launches += graph_kernels[kind];
+        return cudaGraphLaunch(exec, stream);
+      }));
+    } else {
+      for (; launched < max_iter; ++launched) {
+        CK(cudaGraphLaunch(exec, stream));
         launches += graph_kernels[kind];
       }
-      launched += batch;
-      CK(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, stream));
-      CK(cudaStreamSynchronize(stream));
-      if (per_iter && h.niters == launched) {
-        float a = 0, b2 = 0, c = 0;
-        CK(cudaEventElapsedTime(&a, phase[kind][0], phase[kind][1]));
-        CK(cudaEventElapsedTime(&b2, phase[kind][1], phase[kind][2]));
-        CK(cudaEventElapsedTime(&c, phase[kind][2], phase[kind][3]));
-        float d = 0;
-        CK(cudaEventElapsedTime(&d, phase[kind][3], phase[kind][4]));
-        t_mg += a * 1e-3;
-        t_vec += (b2 + d) * 1e-3;
-        t_spmv += c * 1e-3;
-        TRY(read_probes(kind));
-      }
-      if (h.done) break;
     }
-    if (launched == 0) {
-      // max_iter == 0: no iteration ran, but the initial residual norm is
-      // still a result (src/CG.cpp:89-96 sets normr and normr0 before the loop)
+    if (launched == 0 || (!timed && !(tol > 0.0))) {
+      // nothing was read back yet.  max_iter == 0: no iteration ran, but the
+      // initial residual norm is still a result (src/CG.cpp:89-96 sets normr
+      // and normr0 before the loop)
       CK(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, stream));
     }
     // the last iteration's x += alpha p, deferred by k_cg_p
@@ -866,7 +887,8 @@ hpcgx_problem::~hpcgx_problem() {
     cudaEventDestroy(pr.b);
   }
   for (int k = 0; k < G_COUNT; ++k) {
-    if (graph[k]) cudaGraphExecDestroy(graph[k]);
+    for (cudaGraphExec_t exec : graph[k])
+      if (exec) cudaGraphExecDestroy(exec);
     for (int i = 0; i < 5; ++i)
       if (phase[k][i]) cudaEventDestroy(phase[k][i]);
   }
@@ -2138,7 +2160,7 @@ int hpcgx_iteration_bytes(hpcgx_problem *p, int mode, double *bytes) {
   if (!bytes) return fail(HPCGX_EINVAL, "null output");
   int kind = 0;
   TRY(group_kind(mode, &kind));
-  if (!p->graph[kind]) return fail(HPCGX_ESTATE, "no solve of this mode has run on the problem yet");
+  if (!p->graph[kind][0] && !p->graph[kind][1]) return fail(HPCGX_ESTATE, "no solve of this mode has run on the problem yet");
   *bytes = p->graph_bytes[kind];
   return HPCGX_OK;
 }
