@@ -952,34 +952,80 @@ k_prolong(int64_t nc, int nxf, int nyf, const T *__restrict__ xc, T *xf,
 
 // ---------------------------------------------------------------- vectors
 
-__global__ void __launch_bounds__(kThreads)
-k_waxpby(int64_t n, double alpha, const double *__restrict__ x, double beta,
-         const double *__restrict__ y, double *w, const int *__restrict__ done) {
-  if (done && *done) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  // The three branches of src/ComputeWAXPBY_ref.cpp:52-67 round differently.
-  if (alpha == 1.0) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-      w[i] = rn_add(x[i], rn_mul(beta, y[i]));
-  } else if (beta == 1.0) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-      w[i] = rn_add(rn_mul(alpha, x[i]), y[i]);
+// The vector kernels are bound by HBM (or by L2, where the vectors fit it).  A
+// block takes tiles of kTile elements; a thread handles four of a tile, two
+// neighbouring ones and the two half a tile on, with one vector load each, so
+// that a warp's load is one segment and a thread has two loads per vector under
+// way (wide: every vector starts on a two-element boundary).  One element per
+// thread and step before: k_cg_xr at 384^3 331 us -> 270 (5.9 TB/s), a mixed
+// iteration 5.79 -> 5.71 ms; at 64^3 127 -> 123 us.
+constexpr int kVec = 4;
+constexpr int kTile = kVec * kThreads;
+template <int N>
+struct Width {
+  static constexpr int value = N;
+};
+// Runs body(i, width) over [0, n): width 4 for a thread's elements i, i + 1 and
+// i + kTile / 2, i + kTile / 2 + 1 of a tile, width 1 for element i alone.
+template <class F>
+__device__ __forceinline__ void sweep(int64_t n, bool wide, F body) {
+  const int64_t tiles = wide ? n / kTile : 0;
+  for (int64_t b = blockIdx.x; b < tiles; b += gridDim.x)
+    body(b * kTile + 2 * (int)threadIdx.x, Width<kVec>());
+  for (int64_t i = tiles * kTile + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    body(i, Width<1>());
+}
+template <int N, class T>
+__device__ __forceinline__ void get(Width<N>, const T *p, int64_t i, T *v) {
+  if (N == kVec) {
+    load2(p + i, v[0], v[1]);
+    load2(p + i + kTile / 2, v[2], v[3]);
   } else {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-      w[i] = rn_add(rn_mul(alpha, x[i]), rn_mul(beta, y[i]));
+    v[0] = p[i];
   }
+}
+template <int N, class T>
+__device__ __forceinline__ void put(Width<N>, T *p, int64_t i, const T *v) {
+  if (N == kVec) {
+    store2(p + i, v[0], v[1]);
+    store2(p + i + kTile / 2, v[2], v[3]);
+  } else {
+    p[i] = v[0];
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_waxpby(int64_t n, double alpha, const double *x, double beta, const double *y, double *w,
+         int wide, const int *done) {
+  if (done && *done) return;
+  // The three branches of src/ComputeWAXPBY_ref.cpp:52-67 round differently.
+  const int branch = alpha == 1.0 ? 0 : beta == 1.0 ? 1 : 2;
+  sweep(n, wide, [=](int64_t i, auto k) {
+    double a[kVec], b[kVec];
+    get(k, x, i, a);
+    get(k, y, i, b);
+#pragma unroll
+    for (int j = 0; j < k.value; ++j)
+      a[j] = rn_add(branch == 0 ? a[j] : rn_mul(alpha, a[j]), branch == 1 ? b[j] : rn_mul(beta, b[j]));
+    put(k, w, i, a);
+  });
 }
 
 // x.y; the last block stores the total (FIN_STORE into target) or runs a CG
 // scalar step on it (target: the CgState).
 __global__ void __launch_bounds__(kThreads)
-k_dot(int64_t n, const double *__restrict__ x, const double *__restrict__ y, Reduce red, int fin,
-      void *target, const int *__restrict__ done) {
+k_dot(int64_t n, const double *x, const double *y, int wide, Reduce red, int fin, void *target,
+      const int *done) {
   if (done && *done) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   double acc = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-    acc += x[i] * y[i];
+  sweep(n, wide, [&](int64_t i, auto k) {
+    double a[kVec], b[kVec];
+    get(k, x, i, a);
+    get(k, y, i, b);
+#pragma unroll
+    for (int j = 0; j < k.value; ++j) acc += a[j] * b[j];
+  });
   double v[1] = {acc}, tot[1];
   if (grid_reduce<1>(v, red, tot) && threadIdx.x == 0) finish_or_defer<1>(red, fin, target, tot);
 }
@@ -1070,18 +1116,25 @@ k_cg_init(int64_t n, const double *__restrict__ b, const double *__restrict__ Ap
 // rtz = r.z (src/CG.cpp:109/112); for the flexible solver also z.Ap_{k-1}.
 template <class ZT, bool FLEX>
 __global__ void __launch_bounds__(kThreads)
-k_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, Reduce red, CgState *st) {
+k_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, int wide, Reduce red,
+        CgState *st) {
   dependents_launch();
   dependency_wait();
   if (st->done) return;
   const bool two = FLEX && st->k > 1;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   double a0 = 0.0, a1 = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const double zi = (double)z[i];
-    a0 += r[i] * zi;
-    if (two) a1 += zi * Ap[i];
-  }
+  sweep(n, wide, [&](int64_t i, auto k) {
+    double a[kVec], b[kVec];
+    ZT c[kVec];
+    get(k, r, i, a);
+    get(k, z, i, c);
+    if (two) get(k, Ap, i, b);
+#pragma unroll
+    for (int j = 0; j < k.value; ++j) {
+      a0 += a[j] * (double)c[j];
+      if (two) a1 += (double)c[j] * b[j];
+    }
+  });
   if (FLEX) {
     double v[2] = {a0, a1}, tot[2];
     if (grid_reduce<2>(v, red, tot) && threadIdx.x == 0)
@@ -1100,23 +1153,30 @@ k_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, Reduce red, C
 // k_cg_xflush applies the last iteration's update after the loop.
 template <class ZT>
 __global__ void __launch_bounds__(kThreads)
-k_cg_p(int64_t n, const ZT *z, double *p, const CgState *st, double *x) {
+k_cg_p(int64_t n, const ZT *z, double *p, int wide, const CgState *st, double *x) {
   dependents_launch();
   dependency_wait();
   if (st->done) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const bool first = st->k == 1;
   const double beta = st->beta, alpha = st->alpha;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const double zi = (double)z[i];
-    if (first) {
-      p[i] = zi;
-    } else {
-      const double pi = p[i];
-      if (x) x[i] = rn_add(x[i], rn_mul(alpha, pi));
-      p[i] = rn_add(zi, rn_mul(beta, pi));
+  sweep(n, wide, [=](int64_t i, auto k) {
+    double a[kVec], b[kVec];
+    ZT c[kVec];
+    get(k, z, i, c);
+    if (!first) {
+      get(k, (const double *)p, i, a);
+      if (x) {
+        get(k, (const double *)x, i, b);
+#pragma unroll
+        for (int j = 0; j < k.value; ++j) b[j] = rn_add(b[j], rn_mul(alpha, a[j]));
+        put(k, x, i, b);
+      }
     }
-  }
+#pragma unroll
+    for (int j = 0; j < k.value; ++j)
+      a[j] = first ? (double)c[j] : rn_add((double)c[j], rn_mul(beta, a[j]));
+    put(k, p, i, a);
+  });
 }
 
 // The deferred x += alpha p of the last iteration that ran.
@@ -1133,21 +1193,35 @@ k_cg_xflush(int64_t n, const double *__restrict__ p, double *x, const CgState *_
 // (src/CG.cpp:121-124).  r32 (mixed solver): the FP32 copy of r that the
 // V-cycle's finest level reads -- the value it would round r to itself.
 __global__ void __launch_bounds__(kThreads)
-k_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32,
+k_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32, int wide,
         Reduce red, CgState *st) {
   dependents_launch();
   dependency_wait();
   if (st->done) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const double alpha = st->alpha, malpha = -st->alpha;
   double acc = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    if (x) x[i] = rn_add(x[i], rn_mul(alpha, p[i]));
-    const double ri = rn_add(r[i], rn_mul(malpha, Ap[i]));
-    r[i] = ri;
-    if (r32) r32[i] = (float)ri;
-    acc += ri * ri;
-  }
+  sweep(n, wide, [&](int64_t i, auto k) {
+    double a[kVec], b[kVec];
+    get(k, (const double *)r, i, a);
+    get(k, Ap, i, b);
+    if (x) {
+      double c[kVec], e[kVec];
+      get(k, (const double *)x, i, c);
+      get(k, p, i, e);
+#pragma unroll
+      for (int j = 0; j < k.value; ++j) c[j] = rn_add(c[j], rn_mul(alpha, e[j]));
+      put(k, x, i, c);
+    }
+    float f[kVec];
+#pragma unroll
+    for (int j = 0; j < k.value; ++j) {
+      a[j] = rn_add(a[j], rn_mul(malpha, b[j]));
+      f[j] = (float)a[j];
+      acc += a[j] * a[j];
+    }
+    put(k, r, i, a);
+    if (r32) put(k, r32, i, f);
+  });
   double v[1] = {acc}, tot[1];
   if (grid_reduce<1>(v, red, tot) && threadIdx.x == 0)
     finish_or_defer<1>(red, FIN_CG_RR, st, tot);
@@ -1466,9 +1540,13 @@ CgMonitor::~CgMonitor() {
   if (slots) cudaFreeHost(slots);
 }
 
+// Blocks of a vector kernel, a tile each at least.  Up to eight per SM to stream
+// from HBM (25 mixed iterations at 384^3: 5.71 ms each, with four 5.77), four
+// where the vectors stay in L2 and the reduction over the blocks counts (104^3:
+// 237.5 us against 233.7, 128^3: 322 against 317).
 int vector_blocks(int64_t n) {
-  int64_t b = (n + kThreads * 4 - 1) / (kThreads * 4);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * 8));
+  const int64_t b = (n + kTile - 1) / kTile;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * (n > (1 << 23) ? 8 : 4)));
 }
 
 void plan_level(LevelDev &L, int nx, int ny, int nz) {
@@ -1744,21 +1822,27 @@ template int launch_gs_class<float, float>(const LevelDev &, int, int, int, cons
                                            float *, const float *, float *, const int *,
                                            cudaStream_t, int, int);
 
+// Two-element access to every vector of a kernel (null: not used).
+template <class... T>
+int all_aligned2(const T *...v) {
+  return (aligned2(v) && ...);
+}
+
 int launch_waxpby(int64_t n, double alpha, const double *x, double beta, const double *y,
                   double *w, const int *done, cudaStream_t s) {
-  k_waxpby<<<vector_blocks(n), kThreads, 0, s>>>(n, alpha, x, beta, y, w, done);
+  k_waxpby<<<vector_blocks(n), kThreads, 0, s>>>(n, alpha, x, beta, y, w, all_aligned2(x, y, w), done);
   return 1;
 }
 
 int launch_dot(int64_t n, const double *x, const double *y, const Reduce &red, double *out,
                cudaStream_t s) {
-  k_dot<<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, red, FIN_STORE, out, nullptr);
+  k_dot<<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, all_aligned2(x, y), red, FIN_STORE, out, nullptr);
   return 1;
 }
 
 int launch_dot_finish(int64_t n, const double *x, const double *y, const Reduce &red, int fin,
                       CgState *st, cudaStream_t s) {
-  k_dot<<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, red, fin, st, &st->done);
+  k_dot<<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, all_aligned2(x, y), red, fin, st, &st->done);
   return 1;
 }
 
@@ -1806,9 +1890,11 @@ template <class ZT>
 int launch_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, const Reduce &red,
                  CgState *st, cudaStream_t s) {
   if (Ap)
-    launch_dependent(k_cg_rz<ZT, true>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap, red, st);
+    launch_dependent(k_cg_rz<ZT, true>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap,
+                     all_aligned2(r, z, Ap), red, st);
   else
-    launch_dependent(k_cg_rz<ZT, false>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap, red, st);
+    launch_dependent(k_cg_rz<ZT, false>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap,
+                     all_aligned2(r, z, Ap), red, st);
   return 1;
 }
 template int launch_cg_rz<double>(int64_t, const double *, const double *, const double *,
@@ -1818,7 +1904,8 @@ template int launch_cg_rz<float>(int64_t, const double *, const float *, const d
 
 template <class ZT>
 int launch_cg_p(int64_t n, const ZT *z, double *p, CgState *st, cudaStream_t s, double *x) {
-  launch_dependent(k_cg_p<ZT>, dim3(vector_blocks(n)), dim3(kThreads), s, n, z, p, st, x);
+  launch_dependent(k_cg_p<ZT>, dim3(vector_blocks(n)), dim3(kThreads), s, n, z, p,
+                   all_aligned2(z, p, x), st, x);
   return 1;
 }
 template int launch_cg_p<double>(int64_t, const double *, double *, CgState *, cudaStream_t,
@@ -1833,7 +1920,8 @@ int launch_cg_xflush(int64_t n, const double *p, double *x, const CgState *st, c
 
 int launch_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32,
                  const Reduce &red, CgState *st, cudaStream_t s) {
-  launch_dependent(k_cg_xr, dim3(vector_blocks(n)), dim3(kThreads), s, n, p, Ap, x, r, r32, red, st);
+  launch_dependent(k_cg_xr, dim3(vector_blocks(n)), dim3(kThreads), s, n, p, Ap, x, r, r32,
+                   all_aligned2(p, Ap, x, r, r32), red, st);
   return 1;
 }
 
