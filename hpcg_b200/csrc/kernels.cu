@@ -863,6 +863,28 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
   }
 }
 
+// Brings the values of the lines [j0, j1) of a class into L2: whole slices, one
+// bulk prefetch per colour.  The large BF16 classes (three blocks per SM) wait
+// for the latency of their loads more than for HBM; with the values of the block
+// kAhead launches on under way they wait for L2's instead: mixed V-cycle at 384^3
+// 2953 -> 2827 us, at 256^3 941 -> 923 (twice and four times the distance: 2829
+// and 2854; ten times: 2947).  The FP64 sweeps, which HBM bounds, only lose by it
+// (256^3: 2317 -> 2628), and so would a zero-guess sweep that skips most slots.
+constexpr int kAhead = 222;
+template <class VT>
+__device__ __forceinline__ void prefetch_lines(const LevelMat<VT> &A, const ClassInfo &C, int j0,
+                                               int j1) {
+#pragma unroll
+  for (int px = 0; px < 2; ++px) {
+    const int64_t ka = C.start[px] + (int64_t)j0 * C.len[px];
+    const int64_t kb = C.start[px] + (int64_t)j1 * C.len[px];
+    if (kb <= ka) continue;
+    const VT *from = A.vals + (ka >> 5) * kSliceElems;
+    const uint32_t bytes = (uint32_t)((((kb - 1) >> 5) - (ka >> 5) + 1) * kSliceElems * sizeof(VT));
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"(bytes) : "memory");
+  }
+}
+
 // A half sweep over the lines [jbeg, jend) of a class, lpb lines per block (a
 // sharded sweep splits its first launch into the lines that read no halo plane
 // and the rest).  Q >= 0 fixes the class at compile time, which lets the
@@ -891,6 +913,11 @@ k_gs_class(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ Class
   __shared__ T sh[kThreads + 2];
   dependents_launch();
   const int j0 = jbeg + blockIdx.x * lpb;
+  if (MINB == 3 && (!ZERO || (MODE & GS_SYM3)) && threadIdx.x == 0) {
+    if (blockIdx.x < kAhead) prefetch_lines(A, C, j0, min(j0 + lpb, jend));
+    const int jn = j0 + kAhead * lpb;
+    if (jn < jend) prefetch_lines(A, C, jn, min(jn + lpb, jend));
+  }
   gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0, MINB != 3>(
       A, C, 2 * (Q >= 0 ? Q : C.q), j0, min(j0 + lpb, jend), false, (MODE & GS_PROLONG) != 0,
       (MODE & GS_RESTRICT) != 0, !GEN || vec, GEN && A.holes, r, x, xc, rc, sh, done);
