@@ -1376,7 +1376,10 @@ __global__ void k_coarsen_varcoef(Geo gf, Geo gc, int64_t storage_rows_c,
     for (int s = 0; s < HPCGX_STENCIL; ++s) {
       if (s == HPCGX_DIAG_SLOT) continue;
       int64_t col;
-      if (!neighbour(gc, ix, iy, iz, s, row, col)) continue;
+      if (!neighbour(gc, ix, iy, iz, s, row, col)) {
+        cvals[vidx(k, s)] = 0.0;
+        continue;
+      }
       int lx = ix, ly = iy, lz = iz, sl = s;
       if (s < HPCGX_DIAG_SLOT) {
         lx = ix + (s % 3 - 1);
@@ -1394,53 +1397,122 @@ __global__ void k_coarsen_varcoef(Geo gf, Geo gc, int64_t storage_rows_c,
   }
 }
 
-// BF16 copy of the FP64 values (the two arrays group slots differently).
-__global__ void k_to_bf16(int64_t m, const double *__restrict__ v, uint16_t *h) {
+// BF16 copy of the FP64 values (the two arrays group slots differently): a
+// thread converts one z-plane of one storage row, so that a warp reads and
+// writes whole segments of a slice.  Bound by HBM (8 B read, 2 B written per
+// slot); all levels of 192 x 160 x 96: 395 us with a thread per slot, 151 so.
+__global__ void __launch_bounds__(kThreads)
+k_to_bf16(int64_t rows, const double *__restrict__ v, uint16_t *__restrict__ h) {
+  const int64_t m = rows * 3;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = i / HPCGX_STENCIL;
-    const int s = (int)(i - k * HPCGX_STENCIL);
-    h[cidx(k, s)] = bf16_from_double(v[vidx(k, s)]);
+    // 32 rows of a slice side by side, plane by plane
+    const int64_t k = i / 96 * 32 + (i & 31);
+    const int p = (int)(i / 32 % 3);
+    double a[9];
+    load_plane(v, k, p, NeedAll(), a);
+    uint32_t c[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) c[j] = bf16_from_double(a[j]);
+    uint16_t *w = h + (k >> 5) * kSliceElems + p * kPlaneElems;
+    const int lane = (int)(k & 31);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      *reinterpret_cast<uint2 *>(w + j * 128 + lane * 4) =
+          make_uint2(c[4 * j] | c[4 * j + 1] << 16, c[4 * j + 2] | c[4 * j + 3] << 16);
+    w[256 + lane] = (uint16_t)c[8];
   }
+}
+
+// The row-major arrays of 27 slots per natural row (set_values, get_values,
+// adjoint_grad) are read and written by blocks of kTileRows consecutive rows,
+// one segment of kTileRows x 216 B each: a thread per row touched them 216 B
+// apart (set_values at 128^3: 300 us, 229 so).  What a block needs to know of its
+// rows:
+constexpr int kTileRows = 64;
+struct TileRows {
+  int64_t k[kTileRows];      // storage row
+  uint32_t nb[kTileRows];    // bit s: the neighbour of slot s exists
+};
+__device__ __forceinline__ void tile_rows(const Geo &g, int64_t row0, int m, TileRows &t) {
+  for (int i = threadIdx.x; i < m; i += blockDim.x) {
+    const uint32_t row = (uint32_t)row0 + i, nx = g.nx, ny = g.ny;   // fewer than 2^31 rows
+    const uint32_t line = row / nx, ix = row - line * nx, iz = line / ny, iy = line - iz * ny;
+    // bits of a line's three slots, then of a plane's lines, then of the planes
+    const uint32_t x = (ix > 0) | 2u | (uint32_t)(ix + 1 < nx) << 2;
+    const uint32_t y = (iy > 0 ? x : 0u) | x << 3 | (iy + 1 < ny ? x << 6 : 0u);
+    t.nb[i] = (iz > 0 || g.zlo ? y : 0u) | y << 9 | ((int)iz + 1 < g.nz || g.zhi ? y << 18 : 0u);
+    const int px = ix & 1, q = (iy & 1) + 2 * (iz & 1);
+    t.k[i] = g.cstart[px + 2 * q] + ((int64_t)(iz >> 1) * g.nyq[q] + (iy >> 1)) * g.len[px] + (ix >> 1);
+  }
+}
+// Row i of a tile for the i-th of kTileRows neighbouring threads: the even rows,
+// then the odd ones, each a run of storage rows where nx is even.
+__device__ __forceinline__ int tile_row(int i) {
+  return i < kTileRows / 2 ? 2 * i : 2 * (i - kTileRows / 2) + 1;
+}
+__device__ __forceinline__ int64_t slot_column(const Geo &g, int64_t row, int s) {
+  return row + (int64_t)(s / 9 - 1) * g.nx * g.ny + (int64_t)((s / 3) % 3 - 1) * g.nx + (s % 3 - 1);
 }
 
 // Values in natural row order, 27 stencil slots per row -> device layout.
 // Slots without a neighbour stay 0 whatever the input holds.
-__global__ void k_set_values(Geo g, int64_t n, const double *__restrict__ in, double *vals) {
-  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
-       row += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = natural_to_storage(g, row);
-    const int ix = (int)(row % g.nx), iy = (int)((row / g.nx) % g.ny),
-              iz = (int)(row / ((int64_t)g.nx * g.ny));
-    for (int s = 0; s < HPCGX_STENCIL; ++s) {
-      int64_t col;
-      const bool has = neighbour(g, ix, iy, iz, s, row, col);
-      vals[vidx(k, s)] = has ? in[row * HPCGX_STENCIL + s] : 0.0;
-    }
+__global__ void __launch_bounds__(kThreads)
+k_set_values(Geo g, int64_t n, const double *__restrict__ in, double *__restrict__ vals) {
+  __shared__ TileRows t;
+  __shared__ double sh[kTileRows * HPCGX_STENCIL];
+  const int64_t row0 = (int64_t)blockIdx.x * kTileRows;
+  const int m = (int)min((int64_t)kTileRows, n - row0);
+  tile_rows(g, row0, m, t);
+  for (int i = threadIdx.x; i < m * HPCGX_STENCIL; i += blockDim.x)
+    sh[i] = in[row0 * HPCGX_STENCIL + i];
+  __syncthreads();
+  // a plane's slots go out in pairs and one single (vidx): 5 groups a plane
+  for (int i = threadIdx.x; i < 15 * kTileRows; i += blockDim.x) {
+    const int r = tile_row(i % kTileRows), group = i / kTileRows;
+    if (r >= m) continue;
+    const int s = group / 5 * 9 + group % 5 * 2;
+    const uint32_t nb = t.nb[r] >> s;
+    const double *v = sh + r * HPCGX_STENCIL + s;
+    double *to = vals + vidx(t.k[r], s);
+    const double v0 = nb & 1u ? v[0] : 0.0;
+    if (group % 5 < 4)
+      store2(to, v0, nb & 2u ? v[1] : 0.0);
+    else
+      *to = v0;
   }
 }
 
-// The column of (row, s): the neighbour, or the row itself where it has none or
-// the matrix leaves the entry out (holes, value 0).
-__device__ __forceinline__ int64_t column(const Geo &g, int ix, int iy, int iz, int s, int64_t row,
-                                          double v) {
-  int64_t col;
-  const bool has = neighbour(g, ix, iy, iz, s, row, col);
-  return has && !(g.holes && v == 0.0) ? col : row;
-}
-
-__global__ void k_get_values(Geo g, int64_t n, const double *__restrict__ vals, double *out,
-                             int32_t *cout) {
-  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
-       row += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = natural_to_storage(g, row);
-    const int ix = (int)(row % g.nx), iy = (int)((row / g.nx) % g.ny),
-              iz = (int)(row / ((int64_t)g.nx * g.ny));
-    for (int s = 0; s < HPCGX_STENCIL; ++s) {
-      const double v = vals[vidx(k, s)];
-      if (out) out[row * HPCGX_STENCIL + s] = v;
-      if (cout) cout[row * HPCGX_STENCIL + s] = (int32_t)column(g, ix, iy, iz, s, row, v);
-    }
+// Device layout -> natural row order; the column of a slot is its neighbour, or
+// the row itself where it has none or the matrix leaves the entry out (holes,
+// value 0).
+__global__ void __launch_bounds__(kThreads)
+k_get_values(Geo g, int64_t n, const double *__restrict__ vals, double *__restrict__ out,
+             int32_t *__restrict__ cout) {
+  __shared__ TileRows t;
+  __shared__ double sh[kTileRows * HPCGX_STENCIL];
+  const int64_t row0 = (int64_t)blockIdx.x * kTileRows;
+  const int m = (int)min((int64_t)kTileRows, n - row0);
+  tile_rows(g, row0, m, t);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 15 * kTileRows; i += blockDim.x) {
+    const int r = tile_row(i % kTileRows), group = i / kTileRows;
+    if (r >= m) continue;
+    const int s = group / 5 * 9 + group % 5 * 2;
+    double *v = sh + r * HPCGX_STENCIL + s;
+    const double *from = vals + vidx(t.k[r], s);
+    if (group % 5 < 4)
+      load2(from, v[0], v[1]);
+    else
+      v[0] = *from;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < m * HPCGX_STENCIL; i += blockDim.x) {
+    const int r = i / HPCGX_STENCIL, s = i - r * HPCGX_STENCIL;
+    const int64_t row = row0 + r;
+    const bool has = (t.nb[r] >> s & 1u) && !(g.holes && sh[i] == 0.0);
+    if (out) out[row0 * HPCGX_STENCIL + i] = sh[i];
+    if (cout) cout[row0 * HPCGX_STENCIL + i] = (int32_t)(has ? slot_column(g, row, s) : row);
   }
 }
 
@@ -1461,22 +1533,28 @@ __global__ void k_get_diagonal(Geo g, int64_t n, const double *__restrict__ vals
 }
 
 // dL/da_ij = -lambda_i x_j for every stored slot, natural row order, 27 slots
-// per row (zero where the stencil has no neighbour).
-__global__ void k_adjoint_grad(Geo g, int64_t n, const double *__restrict__ vals,
-                               const double *__restrict__ lambda, const double *__restrict__ x,
-                               double *grad) {
-  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
-       row += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = natural_to_storage(g, row);
-    const int ix = (int)(row % g.nx), iy = (int)((row / g.nx) % g.ny),
-              iz = (int)(row / ((int64_t)g.nx * g.ny));
-    const double li = lambda[row];
-    for (int s = 0; s < HPCGX_STENCIL; ++s) {
-      int64_t col;
-      const bool has = neighbour(g, ix, iy, iz, s, row, col);
-      if (has && g.holes) col = column(g, ix, iy, iz, s, row, vals[vidx(k, s)]);
-      grad[row * HPCGX_STENCIL + s] = has ? -(li * x[col]) : 0.0;
+// per row (zero where the stencil has no neighbour).  A thread per slot: the
+// 216 B written per row are the bound (128^3: 646 us with a thread per row, 152
+// so).
+__global__ void __launch_bounds__(kThreads)
+k_adjoint_grad(Geo g, int64_t n, const double *__restrict__ vals,
+               const double *__restrict__ lambda, const double *__restrict__ x,
+               double *__restrict__ grad) {
+  __shared__ TileRows t;
+  const int64_t row0 = (int64_t)blockIdx.x * kTileRows;
+  const int m = (int)min((int64_t)kTileRows, n - row0);
+  tile_rows(g, row0, m, t);
+  __syncthreads();
+  for (int i = threadIdx.x; i < m * HPCGX_STENCIL; i += blockDim.x) {
+    const int r = i / HPCGX_STENCIL, s = i - r * HPCGX_STENCIL;
+    const int64_t row = row0 + r;
+    double v = 0.0;
+    if (t.nb[r] >> s & 1u) {
+      // a left-out entry's column is the row itself
+      const bool hole = g.holes && vals[vidx(t.k[r], s)] == 0.0;
+      v = -(lambda[row] * x[hole ? row : slot_column(g, row, s)]);
     }
+    grad[row0 * HPCGX_STENCIL + i] = v;
   }
 }
 
@@ -1497,6 +1575,8 @@ Geo geo_of(const LevelDev &L) {
   for (int q = 0; q < 4; ++q) g.nyq[q] = L.cls[q].nyq;
   return g;
 }
+
+int tiles_for(int64_t n) { return (int)((n + kTileRows - 1) / kTileRows); }
 
 int grid_for(int64_t n, int threads = kThreads) {
   int64_t b = (n + threads - 1) / threads;
@@ -1637,18 +1717,17 @@ int launch_coarsen_varcoef(const LevelDev &F, const LevelDev &Cc, cudaStream_t s
 }
 
 int launch_to_bf16(const LevelDev &L, cudaStream_t s) {
-  const int64_t m = L.storage_rows * HPCGX_STENCIL;
-  k_to_bf16<<<grid_for(m), kThreads, 0, s>>>(m, L.vals, L.vals16);
+  k_to_bf16<<<grid_for(L.storage_rows * 3), kThreads, 0, s>>>(L.storage_rows, L.vals, L.vals16);
   return 1;
 }
 
 int launch_set_values(const LevelDev &L, const double *vals27, cudaStream_t s) {
-  k_set_values<<<grid_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, vals27, L.vals);
+  k_set_values<<<tiles_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, vals27, L.vals);
   return 1;
 }
 
 int launch_get_values(const LevelDev &L, double *vals27, int32_t *cols27, cudaStream_t s) {
-  k_get_values<<<grid_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, vals27, cols27);
+  k_get_values<<<tiles_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, vals27, cols27);
   return 1;
 }
 
@@ -1959,7 +2038,7 @@ int launch_copy_z(int64_t n, const double *r, double *z, const CgState *st, cuda
 
 int launch_adjoint_grad(const LevelDev &L, const double *lambda, const double *x, double *grad,
                         cudaStream_t s) {
-  k_adjoint_grad<<<grid_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, lambda, x, grad);
+  k_adjoint_grad<<<tiles_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, lambda, x, grad);
   return 1;
 }
 
