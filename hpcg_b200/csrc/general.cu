@@ -21,6 +21,11 @@ int set_error(int code, const char *msg);
 namespace {
 
 constexpr int kT = 256;
+// Rows up to which a level is one block's (k_gen_small).  Solves of the renumbered
+// HPCG hierarchy, ms, without / up to 300 / 2000 / 4096 rows: 48^3 27.4 / 27.0 /
+// 24.9 / 24.6, 32^3 15.4 / 14.8 / 13.2 / 14.1, 16^3 6.5 / 5.9 / 5.1 / 5.5 (where a
+// level has 4096); up to 14000 rows, 48^3 takes 39.
+constexpr int64_t kSmallRows = 2048;
 
 // ------------------------------------------------------------------ kernels
 
@@ -172,6 +177,96 @@ __global__ void k_gen_zero(int64_t n, double *x, const int *done) {
     x[i] = 0.0;
 }
 
+// ---- the small levels of a V-cycle in one block and one launch
+//
+// Below a few thousand rows a colour launch is bound by its latency, some 3 us
+// whatever it updates, and a level has a launch per colour and direction.  One
+// block walks through the colours with a block barrier between them; a thread
+// has the entries of its row of the next colour in registers before it waits.
+struct GenSmallLevel {
+  GenMat A;
+  int ncolors;
+  const int64_t *cstart;
+  const double *r;
+  double *x;
+  int64_t nc;
+  const int32_t *f2c, *f2k;
+};
+struct GenSmallArgs {
+  int n;
+  GenSmallLevel l[kMaxLevels];
+};
+
+__device__ __forceinline__ void gen_update(const GenMat &A, GenRow &w, double d, double r,
+                                           double *x) {
+  const double xi = x[w.i];
+  double sum = r;
+  gen_sum(A, w, x, [&](double v, double xj) { sum = __dsub_rn(sum, __dmul_rn(v, xj)); });
+  sum = __dadd_rn(sum, __dmul_rn(xi, d));
+  x[w.i] = __ddiv_rn(sum, d);
+}
+
+__global__ void __launch_bounds__(kT, 1)
+k_gen_small(const __grid_constant__ GenSmallArgs a, const int *done) {
+  __shared__ int cs[kT + 1];   // colour starts of the level (a row has at most 255 entries)
+  dependents_launch();
+  dependency_wait();
+  if (done && *done) return;
+  const int t = threadIdx.x, last = a.n - 1;
+#pragma unroll 1
+  for (int s = 0; s <= 2 * last; ++s) {
+    const bool down = s <= last;
+    const GenSmallLevel &L = a.l[down ? s : 2 * last - s];
+    const int n = (int)L.A.n, nc = (int)L.nc, C = L.ncolors;
+    for (int c = t; c <= C; c += kT) cs[c] = (int)L.cstart[c];
+    if (down) {
+      for (int i = t; i < n; i += kT) L.x[i] = 0.0;
+    } else {
+      const double *xc = (&L)[1].x;
+      for (int i = t; i < nc; i += kT) L.x[L.f2c[i]] = __dadd_rn(L.x[L.f2c[i]], xc[i]);
+    }
+    __syncthreads();
+    GenRow w;
+    double d = 1.0, r = 0.0;
+    auto fetch = [&](int c) {
+      const int k = cs[c] + t;
+      w.m = 0;
+      if (k >= cs[c + 1]) return;
+      gen_begin(L.A, k, w);
+      d = __ldg(L.A.diag + k);
+      r = L.r[w.i];
+    };
+    fetch(0);
+    // colours 0 .. C-1, then C-1 .. 0
+#pragma unroll 1
+    for (int e = 0; e < 2 * C; ++e) {
+      const int c = e < C ? e : 2 * C - 1 - e;
+      if (w.m > 0) gen_update(L.A, w, d, r, L.x);
+      for (int k = cs[c] + t + kT; k < cs[c + 1]; k += kT) {
+        GenRow o;
+        gen_begin(L.A, k, o);
+        gen_update(L.A, o, L.A.diag[k], L.r[o.i], L.x);
+      }
+      if (e + 1 == 2 * C) break;
+      // the last colour forward and the first one backward are the same rows,
+      // which this thread updates both times (from their first chunk on)
+      if (e + 1 != C) fetch(e + 1 < C ? e + 1 : 2 * C - 2 - e);
+      else if (w.m > kChunk) gen_load(L.A, w, 0);
+      if (e + 1 != C) __syncthreads();
+    }
+    __syncthreads();
+    if (down && s < last) {
+      double *rc = const_cast<double *>((&L)[1].r);
+      for (int i = t; i < nc; i += kT) {
+        GenRow o;
+        gen_begin(L.A, L.f2k[i], o);
+        rc[i] = __dsub_rn(L.r[o.i], gen_product(L.A, o, L.x));
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // Writes (set) or reads the diagonal of every row, natural order.
 __global__ void k_gen_diag(int64_t n, const int64_t *__restrict__ slice_off,
                            const int32_t *__restrict__ perm, const uint8_t *__restrict__ dpos,
@@ -221,6 +316,7 @@ struct GLevel {
   int64_t n = 0, nc = 0, entries = 0;
   int ncolors = 0;
   std::vector<int64_t> cstart;     // storage row of the first row of each colour (+ end)
+  int64_t *dcstart = nullptr;      // the same on the device
   int64_t *slice_off = nullptr;
   uint8_t *nnz = nullptr, *dpos = nullptr;
   int32_t *perm = nullptr, *cols = nullptr, *f2c = nullptr;
@@ -291,9 +387,30 @@ struct GeneralProblem {
     for (int c = 0; c < A.ncolors; ++c) colour(c);
     for (int c = A.ncolors - 1; c >= 0; --c) colour(c);
   }
+  // The first of the small levels, and their part of the V-cycle.
+  int small_from() const {
+    int l = nlev;
+    while (l > 0 && L[l - 1].n <= kSmallRows && L[l - 1].ncolors <= kT) --l;
+    return l;
+  }
+  void small(int l, const double *r, double *x, const int *done) {
+    GenSmallArgs a;
+    a.n = nlev - l;
+    for (int i = 0; i < a.n; ++i) {
+      const GLevel &A = L[l + i];
+      a.l[i] = GenSmallLevel{A.mat(), A.ncolors, A.dcstart, i ? A.r : r, i ? A.x : x,
+                             A.nc, A.f2c, A.f2k};
+    }
+    launch_dependent(k_gen_small, dim3(1), dim3(kT), stream, a, done);
+    note(1);
+  }
   // src/ComputeMG_ref.cpp:39-63, one pre- and one post-smoothing sweep
   // (src/MGData.hpp:51-52).
   void mg(int l, const double *r, double *x, const int *done) {
+    if (l >= small_from()) {
+      small(l, r, x, done);
+      return;
+    }
     const GLevel &A = L[l];
     launch_dependent(k_gen_zero, dim3(grid(A.n)), dim3(kT), stream, A.n, x, done);
     note(1);
@@ -521,6 +638,7 @@ int general_load_level(GeneralProblem *g, int level, int64_t n, const char *nnz,
   GTRY(g->alloc((void **)&A.nnz, n));
   GTRY(g->alloc((void **)&A.dpos, n));
   GTRY(g->alloc((void **)&A.perm, n * sizeof(int32_t)));
+  GTRY(g->alloc((void **)&A.dcstart, A.cstart.size() * sizeof(int64_t)));
   GTRY(g->alloc((void **)&A.cols, entries * sizeof(int32_t)));
   GTRY(g->alloc((void **)&A.vals, entries * sizeof(double)));
   GTRY(g->alloc((void **)&A.diag, n * sizeof(double)));
@@ -542,6 +660,8 @@ int general_load_level(GeneralProblem *g, int level, int64_t n, const char *nnz,
   GCK(cudaMemcpyAsync(A.slice_off, off.data(), (slices + 1) * sizeof(int64_t),
                       cudaMemcpyHostToDevice, s));
   GCK(cudaMemcpyAsync(A.nnz, hn.data(), n, cudaMemcpyHostToDevice, s));
+  GCK(cudaMemcpyAsync(A.dcstart, A.cstart.data(), A.cstart.size() * sizeof(int64_t),
+                      cudaMemcpyHostToDevice, s));
   GCK(cudaMemcpyAsync(A.dpos, hd.data(), n, cudaMemcpyHostToDevice, s));
   GCK(cudaMemcpyAsync(A.perm, perm.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
   GCK(cudaMemcpyAsync(A.cols, hc, entries * sizeof(int32_t), cudaMemcpyHostToDevice, s));

@@ -81,7 +81,7 @@ def mg(levels, l, r):
 
 
 @pytest.mark.parametrize("sizes,most", [((1,), 1), ((31,), 5), ((33, 7), 27), ((500, 61, 9), 28),
-                                        ((1200, 200), 70)])
+                                        ((1200, 200), 70), ((2049, 2048, 300), 40)])
 def test_rows(sizes, most):
     from hpcg_b200 import Problem
     rng = np.random.default_rng(sum(sizes) + most)
