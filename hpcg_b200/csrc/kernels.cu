@@ -1783,28 +1783,32 @@ struct ValsOf<float> {
   static const uint16_t *get(const LevelDev &L) { return L.vals16; }
 };
 
-// The block of a class launch: whole lines.  FP64: a pair needs some 220
-// registers, so two blocks of 128 threads share an SM and one loads while the
-// other computes (V-cycle at 256^3: 2490 us against 2623 with blocks of 256; 128
-// registers for two blocks of 256 spill: 4061).  BF16: blocks of up to 256.  A
-// class of few lines takes fewer lines per block so that there is a block for
-// each SM twice over (a launch is then bound by one block's latency).
-struct GsBlock {
-  int lines, threads;
-};
-template <class T>
-GsBlock gs_block(const ClassInfo &C) {
-  const int target = std::is_same<T, double>::value ? 128 : kThreads;
-  const int len = C.len[0];
-  const int lines = std::min(std::max(1, target / len), std::max(1, C.lines / (2 * 148)));
-  return {lines, std::min(kThreads, (lines * len + 31) / 32 * 32)};
-}
-
 // Pairs of a class from which the BF16 sweeps give up registers (105 -> 80, a
 // few spilled) for a third block per SM: with several waves of blocks another
 // block hides a block's latency (V-cycle at 384^3 3292 us against 3814), with
 // about one wave it does not come to run (64^3: 218 against 228 us).
 constexpr int64_t kManyPairs = 100000;
+
+// The block of a class launch: whole lines.  FP64: a pair needs some 220
+// registers, so two blocks of 128 threads share an SM and one loads while the
+// other computes (V-cycle at 256^3: 2490 us against 2623 with blocks of 256; 128
+// registers for two blocks of 256 spill: 4061).  BF16: blocks of up to 256; of
+// 128 in a large class whose lines fill them (mixed iteration at 256^3 1728 us
+// against 1757, at 128^3 310 against 315), not where threads would idle or a
+// block would be shorter (lines of 192, 96 and 48 pairs, 384^3: 5630 against
+// 5611).  A class of few lines takes fewer lines per block so that there is a
+// block for each SM twice over (a launch is then bound by one block's latency).
+struct GsBlock {
+  int lines, threads;
+};
+template <class T>
+GsBlock gs_block(const ClassInfo &C) {
+  const int len = C.len[0];
+  const bool fills = (int64_t)C.lines * len > kManyPairs && 128 / len * len >= 120;
+  const int target = std::is_same<T, double>::value || fills ? 128 : kThreads;
+  const int lines = std::min(std::max(1, target / len), std::max(1, C.lines / (2 * 148)));
+  return {lines, std::min(kThreads, (lines * len + 31) / 32 * 32)};
+}
 
 // The class kernels, by blocks per SM and form (k_gs_class).
 template <int MINB, bool GEN, class T, class RT>
