@@ -106,14 +106,8 @@ __host__ __device__ inline int64_t vidx(int64_t k, int s) {
   const int lane = (int)(k & 31);
   return r < 8 ? base + (r >> 1) * 64 + lane * 2 + (r & 1) : base + 256 + lane;
 }
-// Index of (storage row k, slot s) in the BF16 value array: per plane, slots
-// r = 0..7 in interleaved quads, slot r = 8 alone.
-__host__ __device__ inline int64_t cidx(int64_t k, int s) {
-  const int p = s / 9, r = s - 9 * p;
-  const int64_t base = (k >> 5) * kSliceElems + p * kPlaneElems;
-  const int lane = (int)(k & 31);
-  return r < 8 ? base + (r >> 2) * 128 + lane * 4 + (r & 3) : base + 256 + lane;
-}
+// (The BF16 array: per plane, slots r = 0..7 in interleaved quads, slot r = 8
+// alone; RowVals<uint16_t> reads it, k_to_bf16 writes it.)
 
 // Colour of the neighbour in slot s of a row of colour c.
 __host__ __device__ constexpr int slot_mask(int s) {
@@ -175,11 +169,6 @@ void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t 
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// Matrix value -> arithmetic type.
-__device__ __forceinline__ double to_arith(double v, double) { return v; }
-__device__ __forceinline__ float to_arith(uint16_t h, float) {
-  return __uint_as_float(((uint32_t)h) << 16);
-}
 // Vector value -> arithmetic type (the finest level of the mixed V-cycle
 // reads its FP64 right-hand side and rounds it to FP32 where it is read).
 __device__ __forceinline__ double vec_to(double v, double) { return v; }

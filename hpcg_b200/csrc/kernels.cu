@@ -2,16 +2,15 @@
 //
 // All kernels are HBM-bandwidth bound (no step of HPCG's PCG iteration is a
 // dense contraction, so nothing here uses tensor cores).  The design points:
-//   * stencil rows are walked by x-line classes (fixed iy&1, iz&1): a CTA owns
-//     whole x-lines and treats the even-x rows, then the odd-x rows of those
-//     lines, so the vector sectors a line touches are completed by one CTA
-//     while they sit in L2;
+//   * stencil rows are walked by x-line classes (fixed iy&1, iz&1), two rows
+//     (2i, 2i+1) per thread from one set of loads;
 //   * a Gauss-Seidel half sweep is ONE launch per class: the two colours of a
-//     class only depend on each other along x inside a line, so a
-//     __syncthreads between them replaces a second launch; the last class's
-//     forward and backward half sweeps are one launch too (its last colour's
-//     backward update follows its forward update from registers), so a
-//     symmetric sweep is 7 launches instead of 16;
+//     class only depend on each other along x inside a line, so a CTA that owns
+//     whole lines takes both with a __syncthreads between them; the last class's
+//     forward and backward half sweeps are one launch too, so a symmetric sweep
+//     is 7 launches instead of 16;
+//   * launches depend on one another programmatically: a kernel starts under the
+//     end of the one before it and waits before it reads a vector;
 //   * restriction (src/ComputeRestriction_ref.cpp:51) is fused into the last
 //     colour of the pre-smoother's backward sweep and prolongation
 //     (src/ComputeProlongation_ref.cpp:49) into the first colour of the
@@ -344,25 +343,6 @@ __device__ __forceinline__ void load_plane(const double *__restrict__ vals, int6
       const double2 t = __ldg(reinterpret_cast<const double2 *>(q + j * 64 + lane * 2));
       v[2 * j] = t.x;
       v[2 * j + 1] = t.y;
-    }
-  }
-  if (need(9 * p + 8)) v[8] = __ldg(q + 256 + lane);
-}
-
-template <class NEED>
-__device__ __forceinline__ void load_plane(const uint16_t *__restrict__ vals, int64_t k, int p,
-                                           NEED need, uint16_t *v) {
-  const uint16_t *q = vals + (k >> 5) * kSliceElems + p * kPlaneElems;
-  const int lane = (int)(k & 31);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    if (need(9 * p + 4 * j) || need(9 * p + 4 * j + 1) || need(9 * p + 4 * j + 2) ||
-        need(9 * p + 4 * j + 3)) {
-      const uint2 t = __ldg(reinterpret_cast<const uint2 *>(q + j * 128 + lane * 4));
-      v[4 * j] = (uint16_t)(t.x & 0xffffu);
-      v[4 * j + 1] = (uint16_t)(t.x >> 16);
-      v[4 * j + 2] = (uint16_t)(t.y & 0xffffu);
-      v[4 * j + 3] = (uint16_t)(t.y >> 16);
     }
   }
   if (need(9 * p + 8)) v[8] = __ldg(q + 256 + lane);
