@@ -89,9 +89,11 @@ struct LevelMat {
   // that neighbour (the layout enforces it when a level is loaded), and column
   // i with value 0 otherwise.
   int off[HPCGX_STENCIL];
-  // a loaded matrix whose rows leave out entries of existing neighbours: such a
-  // slot (value 0) is column i too
-  int holes;
+  // Which entries of existing neighbours a loaded matrix leaves out: bit s of
+  // left_out[k] is set where storage row k has none in slot s.  Such a slot holds
+  // 0 too, but its column is the row itself, which the value cannot tell (a
+  // stored 0 keeps its column).  Null where no row leaves one out.
+  const uint32_t *left_out;
 };
 
 // Elements of one 32-row slice and of one z-plane inside it.
@@ -112,6 +114,16 @@ __host__ __device__ inline int64_t vidx(int64_t k, int s) {
 // Colour of the neighbour in slot s of a row of colour c.
 __host__ __device__ constexpr int slot_mask(int s) {
   return ((s % 3) != 1 ? 1 : 0) | (((s / 3) % 3) != 1 ? 2 : 0) | ((s / 9) != 1 ? 4 : 0);
+}
+
+// The slots whose neighbour exists, as bits, for a row with (1) or without (0)
+// neighbours at x - 1, x + 1, y - 1, ...: a line's three, then a plane's lines,
+// then the planes.
+__host__ __device__ __forceinline__ uint32_t stencil_bits(bool xm, bool xp, bool ym, bool yp,
+                                                          bool zm, bool zp) {
+  const uint32_t x = (xm ? 1u : 0u) | 2u | (xp ? 4u : 0u);
+  const uint32_t y = (ym ? x : 0u) | x << 3 | (yp ? x << 6 : 0u);
+  return (zm ? y : 0u) | y << 9 | (zp ? y << 18 : 0u);
 }
 
 // Arithmetic with one rounding per operation and no contraction into FMA,

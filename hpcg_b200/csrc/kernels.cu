@@ -427,17 +427,17 @@ struct NeedAll {
 // 32-bit arithmetic: vectors hold fewer than 2^31 rows), the row itself
 // elsewhere and for a left-out entry, so that the product with the slot's 0
 // reads nothing the row does not read anyway.
-template <class VT, class V>
-__device__ __forceinline__ void stencil_cols(const LevelMat<VT> &A, const RowId &id, const V *val,
-                                             int32_t *col) {
+template <class VT>
+__device__ __forceinline__ void stencil_cols(const LevelMat<VT> &A, const RowId &id, int32_t *col) {
   const int r32 = (int)id.row;
+  const uint32_t out = A.left_out ? A.left_out[id.k] : 0u;
   const bool xm = id.ix > 0, xp = id.ix + 1 < A.nx, ym = id.iy > 0, yp = id.iy + 1 < A.ny,
              zm = id.iz > 0 || A.zlo, zp = id.iz + 1 < A.nz || A.zhi;
 #pragma unroll
   for (int s = 0; s < HPCGX_STENCIL; ++s) {
     const int dx = s % 3 - 1, dy = (s / 3) % 3 - 1, dz = s / 9 - 1;
     const bool nb = (dx < 0 ? xm : dx > 0 ? xp : true) && (dy < 0 ? ym : dy > 0 ? yp : true) &&
-                    (dz < 0 ? zm : dz > 0 ? zp : true) && !(A.holes && val[s] == V(0));
+                    (dz < 0 ? zm : dz > 0 ? zp : true) && !(out >> s & 1u);
     col[s] = nb ? r32 + A.off[s] : r32;
   }
 }
@@ -543,15 +543,15 @@ __device__ __forceinline__ void load_line(const LevelMat<VT> &A, const PairId &i
   if (ok && id.right) v[3] = q[2];
 }
 
-// One term of a row sum.  holes: a left-out entry (value 0) adds nothing
-// whatever its neighbour holds (LevelMat::holes).
+// Slot s of a row sum.  out: the row's left-out entries (LevelMat::left_out),
+// which add nothing whatever their neighbour holds; a stored zero multiplies it.
 template <class T>
-__device__ __forceinline__ T term_add(bool holes, T sum, T v, T x) {
-  return holes && v == T(0) ? sum : mac_add(sum, v, x);
+__device__ __forceinline__ T term_add(uint32_t out, int s, T sum, T v, T x) {
+  return out >> s & 1u ? sum : mac_add(sum, v, x);
 }
 template <class T>
-__device__ __forceinline__ T term_sub(bool holes, T sum, T v, T x) {
-  return holes && v == T(0) ? sum : mac_sub(sum, v, x);
+__device__ __forceinline__ T term_sub(uint32_t out, int s, T sum, T v, T x) {
+  return out >> s & 1u ? sum : mac_sub(sum, v, x);
 }
 
 // ---------------------------------------------------------------- SpMV
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kThreads, std::is_same<VT, double>::value ? 2 
 k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet cs, const T *x,
        T *y, int wide, Reduce red, int fin, void *fin_target, const int *done) {
   dependents_launch();
-  const bool vec = !GEN || wide, holes = GEN && A.holes;
+  const bool vec = !GEN || wide;
   int q, b;
   class_block(cs, (int)blockIdx.x, q, b);
   const ClassInfo &C = cs.c[q];
@@ -580,8 +580,13 @@ k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet 
   const bool act = t < C.lines * C.len[0];
   PairId id;
   T ve[9], vo[9];
+  uint32_t oe = 0u, oo = 0u;   // left-out entries of the two rows
   if (act) {
     id = pair_of(A, C, 0, t, 1);
+    if (GEN && A.left_out) {
+      oe = A.left_out[id.ke];
+      oo = A.left_out[id.ko];
+    }
     load_vals(A.vals, id.ke, 0, NeedAll(), ve);
     load_vals(A.vals, id.ko, 0, NeedAll(), vo);
   }
@@ -601,8 +606,8 @@ k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet 
       for (int i = 0; i < 3; ++i) load_line(A, id, xr, 3 * p + i, true, vec, v[i], 2);
 #pragma unroll
       for (int s = 0; s < 9; ++s) {
-        se = term_add(holes, se, ve[s], v[s / 3][s % 3]);
-        so = term_add(holes, so, vo[s], v[s / 3][s % 3 + 1]);
+        se = term_add(oe, 9 * p + s, se, ve[s], v[s / 3][s % 3]);
+        so = term_add(oo, 9 * p + s, so, vo[s], v[s / 3][s % 3 + 1]);
       }
       if (p == 1) {
         xe = v[1][1];
@@ -638,7 +643,8 @@ k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet 
 // soon as it is loaded -- once for a row that is updated twice (class 3) and
 // for the residual that GS_RESTRICT forms -- and only the second part stays in
 // registers over the exchange between the two rows of a pair.
-// PX: the row's place in the pair (0 even, 1 odd); c: its colour.
+// PX: the row's place in the pair (0 even, 1 odd); c: its colour; out: its
+// left-out entries.
 // ZERO: x is zero for every colour above c and for the row itself (first
 //       forward sweep after ZeroVector); those terms are skipped.  Skipping a
 //       product with a zero changes nothing but possibly the sign of an exact
@@ -646,25 +652,26 @@ k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet 
 constexpr int kHead = 12;   // slots of the first part
 
 template <int PX, bool ZERO, class V, class T>
-__device__ __forceinline__ T gs_head(bool holes, int c, const V &val, const T (&xl)[4][4], T sum) {
+__device__ __forceinline__ T gs_head(uint32_t out, int c, const V &val, const T (&xl)[4][4], T sum) {
 #pragma unroll
   for (int s = 0; s < kHead; ++s)
     if (!(ZERO && (c ^ slot_mask(s)) > c))
-      sum = term_sub(holes, sum, (T)val.get(s), xl[s / 3][s % 3 + PX]);
+      sum = term_sub(out, s, sum, (T)val.get(s), xl[s / 3][s % 3 + PX]);
   return sum;
 }
 
 // xl[l - 4][0..3] = x[2i-1 .. 2i+2] of line l; xi: the row's own entry before
 // the update.
 template <int PX, bool ZERO, class V, class T>
-__device__ __forceinline__ T gs_tail(bool holes, int c, const V &val, const T (&xl)[5][4], T sum, T xi) {
+__device__ __forceinline__ T gs_tail(uint32_t out, int c, const V &val, const T (&xl)[5][4], T sum,
+                                     T xi) {
   const T d = val.get(HPCGX_DIAG_SLOT);
 #pragma unroll
   for (int s = kHead; s < HPCGX_STENCIL; ++s) {
     if (s == HPCGX_DIAG_SLOT) {
       if (!ZERO) sum = mac_sub(sum, d, xi);
     } else if (!(ZERO && (c ^ slot_mask(s)) > c)) {
-      sum = term_sub(holes, sum, (T)val.get(s), xl[s / 3 - 4][s % 3 + PX]);
+      sum = term_sub(out, s, sum, (T)val.get(s), xl[s / 3 - 4][s % 3 + PX]);
     }
   }
   if (!ZERO) sum = mac_add(sum, xi, d);
@@ -699,8 +706,8 @@ __device__ __forceinline__ T gs_tail(bool holes, int c, const V &val, const T (&
 template <int DIR, bool ZERO, bool SYM3, bool AHEAD, class VT, class T, class RT>
 __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo &C, int ce, int j0,
                                          int j1, bool zero, bool pro, bool res, bool vec,
-                                         bool holes, const RT *r, T *x, const T *xc, T *rc, T *sh,
-                                         const int *done) {
+                                         const uint32_t *left_out, const RT *r, T *x, const T *xc,
+                                         T *rc, T *sh, const int *done) {
   const int cnt = (j1 - j0) * C.len[0];
   const int nb = blockDim.x, tid = threadIdx.x;
   const int chunks = (cnt + nb - 1) / nb;
@@ -714,6 +721,7 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
     const bool act = t < cnt;
     PairId id;
     RowVals<VT> ve, vo;
+    uint32_t oe = 0u, oo = 0u;
     T xl[5][4];
     T se = T(0), so = T(0), ax = T(0), xe = T(0), xo = T(0), re = T(0);
     int64_t crow = 0;
@@ -723,6 +731,10 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
     }
     if (act) {
       id = pair_of(A, C, j0, t, 3);
+      if (left_out) {
+        oe = left_out[id.ke];
+        oo = left_out[id.ko];
+      }
 #pragma unroll
       for (int p = 0; p < 3; ++p) {
         ve.load(A.vals, id.ke, p, need_e);
@@ -758,11 +770,11 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
           else
             load_line(A, id, xr, l, !zero || there, vec, to, 4);
         }
-        se = gs_head<0, ZERO>(holes, ce, ve, xh, re);
-        so = gs_head<1, ZERO>(holes, co, vo, xh, ro);
+        se = gs_head<0, ZERO>(oe, ce, ve, xh, re);
+        so = gs_head<1, ZERO>(oo, co, vo, xh, ro);
         if (res) {
 #pragma unroll
-          for (int s = 0; s < kHead; ++s) ax = term_add(holes, ax, (T)ve.get(s), xh[s / 3][s % 3]);
+          for (int s = 0; s < kHead; ++s) ax = term_add(oe, s, ax, (T)ve.get(s), xh[s / 3][s % 3]);
         }
       }
       if (pro || res) {
@@ -774,10 +786,10 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
       xo = xl[0][2];
       if (pro && !(A.zlo && id.iz == 0)) xe = rn_add(xe, xc[crow]);
       if (DIR == 0) {
-        xe = gs_tail<0, ZERO>(holes, ce, ve, xl, se, xe);
+        xe = gs_tail<0, ZERO>(oe, ce, ve, xl, se, xe);
         sh[tid] = xe;
       } else if (id.odd) {
-        xo = gs_tail<1, false>(holes, co, vo, xl, so, xo);
+        xo = gs_tail<1, false>(oo, co, vo, xl, so, xo);
         sh[tid + 1] = xo;
       }
     }
@@ -787,21 +799,21 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
         xl[0][1] = xe;
         if (id.right) xl[0][3] = tid + 1 < nb ? sh[tid + 1] : x[id.row + 2];
         if (id.odd) {
-          xo = gs_tail<1, ZERO>(holes, co, vo, xl, so, xo);
+          xo = gs_tail<1, ZERO>(oo, co, vo, xl, so, xo);
           // forward then backward: between the two only the row's own entry
           // changes
-          if (SYM3) xo = gs_tail<1, false>(holes, co, vo, xl, so, xo);
+          if (SYM3) xo = gs_tail<1, false>(oo, co, vo, xl, so, xo);
         }
       } else {
         xl[0][2] = xo;
         if (id.left) xl[0][0] = tid > 0 ? sh[tid] : x[id.row - 1];
-        xe = gs_tail<0, false>(holes, ce, ve, xl, se, xe);
+        xe = gs_tail<0, false>(oe, ce, ve, xl, se, xe);
       }
       if (res) {
 #pragma unroll
         for (int s = kHead; s < HPCGX_STENCIL; ++s)
-          ax = term_add(holes, ax, (T)ve.get(s),
-                               s == HPCGX_DIAG_SLOT ? xe : xl[s / 3 - 4][s % 3]);
+          ax = term_add(oe, s, ax, (T)ve.get(s),
+                        s == HPCGX_DIAG_SLOT ? xe : xl[s / 3 - 4][s % 3]);
         rc[crow] = rn_sub(re, ax);
       }
     }
@@ -812,7 +824,7 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
       if (act) {
         xl[0][2] = xo;
         if (id.left) xl[0][0] = sh[tid];
-        xe = gs_tail<0, false>(holes, ce, ve, xl, se, xe);
+        xe = gs_tail<0, false>(oe, ce, ve, xl, se, xe);
       }
     }
     if (act) {
@@ -837,8 +849,9 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
       for (int l = 0; l < 9; ++l)
         load_line(A, id, (const T *)x + id.row, l, true, vec,
                   l < 4 ? xh[l < 4 ? l : 0] : xl[l < 4 ? 0 : l - 4], 4);
-      const T sum = gs_head<0, false>(holes, ce, ve, xh, vec_to(r[id.row], T()));
-      x[id.row] = gs_tail<0, false>(holes, ce, ve, xl, sum, xl[0][1]);
+      const uint32_t oe = left_out ? left_out[id.ke] : 0u;
+      const T sum = gs_head<0, false>(oe, ce, ve, xh, vec_to(r[id.row], T()));
+      x[id.row] = gs_tail<0, false>(oe, ce, ve, xl, sum, xl[0][1]);
     }
   }
 }
@@ -900,7 +913,7 @@ k_gs_class(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ Class
   }
   gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0, MINB != 3>(
       A, C, 2 * (Q >= 0 ? Q : C.q), j0, min(j0 + lpb, jend), false, (MODE & GS_PROLONG) != 0,
-      (MODE & GS_RESTRICT) != 0, !GEN || vec, GEN && A.holes, r, x, xc, rc, sh, done);
+      (MODE & GS_RESTRICT) != 0, !GEN || vec, GEN ? A.left_out : nullptr, r, x, xc, rc, sh, done);
 }
 
 // Residual restricted at the injected points (colour 0: even ix, iy, iz):
@@ -931,7 +944,7 @@ k_restrict_residual(LevelMat<VT> A, ClassInfo C0, int64_t nc, const RT *__restri
     T val[HPCGX_STENCIL];
 #pragma unroll
     for (int p = 0; p < 3; ++p) load_vals(A.vals, id.k, p, NeedAll(), val + 9 * p);
-    stencil_cols(A, id, val, col);
+    stencil_cols(A, id, col);
     check_cols(A, col, NeedAll(), 7);
     T ax = T(0);
 #pragma unroll
@@ -1247,7 +1260,7 @@ __global__ void k_copy_z(int64_t n, const double *__restrict__ r, double *z,
 struct Geo {
   int nx, ny, nz;
   int zlo, zhi;   // z-slab: the planes below / above belong to a neighbouring rank
-  int holes;      // the matrix leaves out entries of existing neighbours
+  const uint32_t *left_out;   // LevelMat::left_out
   int64_t cstart[8], ccount[8];
   int len[2];
   int nyq[4];
@@ -1418,13 +1431,15 @@ __device__ __forceinline__ void tile_rows(const Geo &g, int64_t row0, int m, Til
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
     const uint32_t row = (uint32_t)row0 + i, nx = g.nx, ny = g.ny;   // fewer than 2^31 rows
     const uint32_t line = row / nx, ix = row - line * nx, iz = line / ny, iy = line - iz * ny;
-    // bits of a line's three slots, then of a plane's lines, then of the planes
-    const uint32_t x = (ix > 0) | 2u | (uint32_t)(ix + 1 < nx) << 2;
-    const uint32_t y = (iy > 0 ? x : 0u) | x << 3 | (iy + 1 < ny ? x << 6 : 0u);
-    t.nb[i] = (iz > 0 || g.zlo ? y : 0u) | y << 9 | ((int)iz + 1 < g.nz || g.zhi ? y << 18 : 0u);
+    t.nb[i] = stencil_bits(ix > 0, ix + 1 < nx, iy > 0, iy + 1 < ny, iz > 0 || g.zlo,
+                           (int)iz + 1 < g.nz || g.zhi);
     const int px = ix & 1, q = (iy & 1) + 2 * (iz & 1);
     t.k[i] = g.cstart[px + 2 * q] + ((int64_t)(iz >> 1) * g.nyq[q] + (iy >> 1)) * g.len[px] + (ix >> 1);
   }
+}
+// Row r of a tile: does the matrix leave out its entry in slot s?
+__device__ __forceinline__ bool left_out(const Geo &g, const TileRows &t, int r, int s) {
+  return g.left_out && (g.left_out[t.k[r]] >> s & 1u);
 }
 // Row i of a tile for the i-th of kTileRows neighbouring threads: the even rows,
 // then the odd ones, each a run of storage rows where nx is even.
@@ -1464,8 +1479,7 @@ k_set_values(Geo g, int64_t n, const double *__restrict__ in, double *__restrict
 }
 
 // Device layout -> natural row order; the column of a slot is its neighbour, or
-// the row itself where it has none or the matrix leaves the entry out (holes,
-// value 0).
+// the row itself where it has none or the matrix leaves the entry out.
 __global__ void __launch_bounds__(kThreads)
 k_get_values(Geo g, int64_t n, const double *__restrict__ vals, double *__restrict__ out,
              int32_t *__restrict__ cout) {
@@ -1490,7 +1504,7 @@ k_get_values(Geo g, int64_t n, const double *__restrict__ vals, double *__restri
   for (int i = threadIdx.x; i < m * HPCGX_STENCIL; i += blockDim.x) {
     const int r = i / HPCGX_STENCIL, s = i - r * HPCGX_STENCIL;
     const int64_t row = row0 + r;
-    const bool has = (t.nb[r] >> s & 1u) && !(g.holes && sh[i] == 0.0);
+    const bool has = (t.nb[r] >> s & 1u) && !left_out(g, t, r, s);
     if (out) out[row0 * HPCGX_STENCIL + i] = sh[i];
     if (cout) cout[row0 * HPCGX_STENCIL + i] = (int32_t)(has ? slot_column(g, row, s) : row);
   }
@@ -1517,9 +1531,8 @@ __global__ void k_get_diagonal(Geo g, int64_t n, const double *__restrict__ vals
 // 216 B written per row are the bound (128^3: 646 us with a thread per row, 152
 // so).
 __global__ void __launch_bounds__(kThreads)
-k_adjoint_grad(Geo g, int64_t n, const double *__restrict__ vals,
-               const double *__restrict__ lambda, const double *__restrict__ x,
-               double *__restrict__ grad) {
+k_adjoint_grad(Geo g, int64_t n, const double *__restrict__ lambda,
+               const double *__restrict__ x, double *__restrict__ grad) {
   __shared__ TileRows t;
   const int64_t row0 = (int64_t)blockIdx.x * kTileRows;
   const int m = (int)min((int64_t)kTileRows, n - row0);
@@ -1531,8 +1544,7 @@ k_adjoint_grad(Geo g, int64_t n, const double *__restrict__ vals,
     double v = 0.0;
     if (t.nb[r] >> s & 1u) {
       // a left-out entry's column is the row itself
-      const bool hole = g.holes && vals[vidx(t.k[r], s)] == 0.0;
-      v = -(lambda[row] * x[hole ? row : slot_column(g, row, s)]);
+      v = -(lambda[row] * x[left_out(g, t, r, s) ? row : slot_column(g, row, s)]);
     }
     grad[row0 * HPCGX_STENCIL + i] = v;
   }
@@ -1545,7 +1557,7 @@ Geo geo_of(const LevelDev &L) {
   g.nz = L.nz;
   g.zlo = L.zlo;
   g.zhi = L.zhi;
-  g.holes = L.holes;
+  g.left_out = L.holes ? L.left_out : nullptr;
   for (int c = 0; c < 8; ++c) {
     g.cstart[c] = L.cstart[c];
     g.ccount[c] = L.ccount[c];
@@ -1578,7 +1590,9 @@ LevelMat<VT> mat_of(const LevelDev &L, const VT *vals) {
   A.lo = L.zlo ? -L.nx * L.ny : 0;
   A.span = (int)L.n - A.lo + (L.zhi ? L.nx * L.ny : 0);
   A.srows = L.storage_rows;
-  A.holes = L.holes;
+  // left-out entries are a matter of the FP64 operators; the BF16 copy
+  // multiplies the neighbour by 0
+  A.left_out = L.holes && std::is_same<VT, double>::value ? L.left_out : nullptr;
   return A;
 }
 
@@ -1796,10 +1810,7 @@ int launch_gs_rows(const LevelDev &L, int q, int backward, int mode, const RT *r
                    const T *xc, T *rc, const int *done, cudaStream_t s, int jbeg, int jend,
                    GsBlock gb, int vec) {
   using VT = typename ValsOf<T>::VT;
-  LevelMat<VT> A = mat_of(L, ValsOf<T>::get(L));
-  // left-out entries are a matter of the FP64 operators; the BF16 copy
-  // multiplies the neighbour by 0
-  if (!std::is_same<T, double>::value) A.holes = 0;
+  const LevelMat<VT> A = mat_of(L, ValsOf<T>::get(L));
   const dim3 g((unsigned)((jend - jbeg + gb.lines - 1) / gb.lines)), b(gb.threads);
   const ClassInfo &C = L.cls[q];
   auto go = [&](auto kernel) {
@@ -2022,7 +2033,7 @@ int launch_copy_z(int64_t n, const double *r, double *z, const CgState *st, cuda
 
 int launch_adjoint_grad(const LevelDev &L, const double *lambda, const double *x, double *grad,
                         cudaStream_t s) {
-  k_adjoint_grad<<<tiles_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, L.vals, lambda, x, grad);
+  k_adjoint_grad<<<tiles_for(L.n), kThreads, 0, s>>>(geo_of(L), L.n, lambda, x, grad);
   return 1;
 }
 

@@ -14,8 +14,10 @@ struct LevelDev {
   int64_t cstart[8] = {}, ccount[8] = {};
   ClassInfo cls[4] = {};
   int spmv_blocks = 0;        // all four classes in one launch
-  // a loaded matrix that leaves out entries of existing neighbours (LevelMat)
+  // a loaded matrix that leaves out entries of existing neighbours: which ones
+  // (LevelMat::left_out; storage_rows words, allocated for such a matrix only)
   bool holes = false;
+  uint32_t *left_out = nullptr;
   // z-slab of a sharded problem: a neighbouring rank owns the plane below
   // (zlo) / above (zhi); vectors read by SpMV and Gauss-Seidel then hold one
   // halo plane on each side (indices -nx*ny..-1 and n..n+nx*ny-1)

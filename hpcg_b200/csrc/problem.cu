@@ -211,15 +211,19 @@ struct hpcgx_problem {
     return HPCGX_OK;
   }
   // ---- pinned host staging of the host loaders: two chunks of kPinnedSlices
-  // 32-row slices of values, allocated on the first load
+  // 32-row slices of values and of left-out bits, allocated on the first load
   double *pin_vals[2] = {};
+  uint32_t *pin_out[2] = {};
   cudaEvent_t pin_copied[2] = {};
   int pinned_staging() {
-    if (pin_vals[0]) return HPCGX_OK;
+    if (pin_copied[1]) return HPCGX_OK;
     const size_t e = (size_t)kPinnedSlices * kSliceElems;
     for (int h = 0; h < 2; ++h) {
-      CK(cudaHostAlloc((void **)&pin_vals[h], e * sizeof(double), cudaHostAllocDefault));
-      CK(cudaEventCreateWithFlags(&pin_copied[h], cudaEventDisableTiming));
+      if (!pin_vals[h]) CK(cudaHostAlloc((void **)&pin_vals[h], e * sizeof(double), cudaHostAllocDefault));
+      if (!pin_out[h])
+        CK(cudaHostAlloc((void **)&pin_out[h], kPinnedSlices * HPCGX_SLICE * sizeof(uint32_t),
+                         cudaHostAllocDefault));
+      if (!pin_copied[h]) CK(cudaEventCreateWithFlags(&pin_copied[h], cudaEventDisableTiming));
     }
     return HPCGX_OK;
   }
@@ -895,6 +899,7 @@ hpcgx_problem::~hpcgx_problem() {
   for (int l = 0; l < kMaxLevels; ++l) {
     cudaFree(L[l].vals);
     cudaFree(L[l].vals16);
+    cudaFree(L[l].left_out);
     cudaFree(L[l].r64);
     cudaFree(L[l].r32);
   }
@@ -903,6 +908,7 @@ hpcgx_problem::~hpcgx_problem() {
   for (int h = 0; h < 2; ++h) {
     if (pin_copied[h]) cudaEventDestroy(pin_copied[h]);
     if (pin_vals[h]) cudaFreeHost(pin_vals[h]);
+    if (pin_out[h]) cudaFreeHost(pin_out[h]);
   }
   for (void *ptr : {(void *)b, (void *)x, (void *)r, (void *)r32, (void *)Ap, (void *)tmp,
                     (void *)result,
@@ -985,12 +991,11 @@ template <class Nnz, class Get>
 int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
   TRY(check_level(p, level));
   LevelDev &A = p->L[level];
-  // One row: validates it and writes its 27 slots through put(s, col, val);
-  // returns an empty string or what is wrong with the row.
+  // One row: validates it and writes its entries through put(s, val); returns an
+  // empty string or what is wrong with the row.
   auto scan_row = [&](int64_t row, auto put) -> std::string {
     const int ix = (int)(row % A.nx), iy = (int)((row / A.nx) % A.ny),
               iz = (int)(row / ((int64_t)A.nx * A.ny));
-    for (int s = 0; s < HPCGX_STENCIL; ++s) put(s, 0.0);
     const int nz = nnz_of(row);
     if (nz < 1 || nz > HPCGX_STENCIL) return std::to_string(nz) + " entries";
     int last = -1;
@@ -1021,9 +1026,7 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
   int64_t off[HPCGX_STENCIL];
   for (int s = 0; s < HPCGX_STENCIL; ++s)
     off[s] = (s % 3 - 1) + (int64_t)A.nx * ((s / 3) % 3 - 1 + (int64_t)A.ny * (s / 9 - 1));
-  std::atomic<bool> holes{false};
   auto fast_row = [&](int64_t row, int ix, int iy, int iz, auto put) -> bool {
-    for (int s = 0; s < HPCGX_STENCIL; ++s) put(s, 0.0);
     const int nz = nnz_of(row);
     if (nz < 1 || nz > HPCGX_STENCIL) return false;
     const bool okx[3] = {ix > 0, true, ix + 1 < A.nx}, oky[3] = {iy > 0, true, iy + 1 < A.ny},
@@ -1042,9 +1045,6 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
       put(s, v);
       ++s;
     }
-    // an existing neighbour without an entry
-    if (nz < (okx[0] + 1 + okx[2]) * (oky[0] + 1 + oky[2]) * (okz[0] + 1 + okz[2]))
-      holes.store(true, std::memory_order_relaxed);
     return diag;
   };
   p->loaded[level] = false;
@@ -1052,11 +1052,13 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
   const int64_t slices = A.storage_rows / HPCGX_SLICE;
   TRY(p->pinned_staging());
   bool pending[2] = {false, false};
-  bool failed = false;
+  bool failed = false, holes = false;
   std::vector<char> bad(64);
   for (int64_t c0 = 0, it = 0; c0 < slices && !failed; c0 += kPinnedSlices, ++it) {
     const int h = (int)(it & 1);
     double *bv = p->pin_vals[h];
+    uint32_t *bo = p->pin_out[h];
+    std::atomic<bool> gone{false};   // a row of this chunk leaves out an entry
     if (pending[h]) CK(cudaEventSynchronize(p->pin_copied[h]));
     pending[h] = false;
     const int64_t c1 = std::min(slices, c0 + kPinnedSlices);
@@ -1065,21 +1067,49 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
       for (int64_t k = k0 + a; k < k0 + e; ++k) {
         int ix, iy, iz;
         const int64_t row = natural_row_host(A, k, ix, iy, iz);
-        if (row < 0) {   // padding
+        uint32_t has = 0u;
+        auto blank = [&]() {
           for (int s = 0; s < HPCGX_STENCIL; ++s) bv[vidx(k, s) - e0] = 0.0;
-          continue;
+          has = 0u;
+        };
+        blank();
+        bo[k - k0] = 0u;
+        if (row < 0) continue;   // padding
+        auto put = [&](int s, double v) {
+          bv[vidx(k, s) - e0] = v;
+          has |= 1u << s;
+        };
+        if (!fast_row(row, ix, iy, iz, put)) {
+          blank();
+          if (!scan_row(row, put).empty()) {
+            bad[t] = 1;
+            return;
+          }
         }
-        auto put = [&](int s, double v) { bv[vidx(k, s) - e0] = v; };
-        if (!fast_row(row, ix, iy, iz, put) && !scan_row(row, put).empty()) {
-          bad[t] = 1;
-          return;
-        }
+        const uint32_t out = ~has & stencil_bits(ix > 0, ix + 1 < A.nx, iy > 0, iy + 1 < A.ny,
+                                                 iz > 0, iz + 1 < A.nz);
+        bo[k - k0] = out;
+        if (out) gone.store(true, std::memory_order_relaxed);
       }
     });
     for (char f : bad) failed |= f != 0;
     if (failed) break;
     const size_t ne = (size_t)(c1 - c0) * kSliceElems;
     CK(cudaMemcpyAsync(A.vals + e0, bv, ne * sizeof(double), cudaMemcpyHostToDevice, p->stream));
+    if (gone.load()) {
+      if (!holes) {   // the chunks before leave nothing out
+        const size_t all = A.storage_rows * sizeof(uint32_t);
+        const int rc = A.left_out ? HPCGX_OK : p->alloc((void **)&A.left_out, all);
+        if (rc != HPCGX_OK) {
+          cudaStreamSynchronize(p->stream);   // the copies from the staging
+          return rc;
+        }
+        CK(cudaMemsetAsync(A.left_out, 0, all, p->stream));
+        holes = true;
+      }
+      CK(cudaMemcpyAsync(A.left_out + k0, bo, (size_t)(c1 - c0) * HPCGX_SLICE * sizeof(uint32_t),
+                         cudaMemcpyHostToDevice, p->stream));
+    }
     CK(cudaEventRecord(p->pin_copied[h], p->stream));
     pending[h] = true;
   }
@@ -1102,7 +1132,7 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
       if (first[t] >= 0) return fail(HPCGX_ELAYOUT, "row " + std::to_string(first[t]) + ": " + msg[t]);
     return fail(HPCGX_ELAYOUT, "malformed row");
   }
-  A.holes = holes.load();
+  A.holes = holes;
   p->loaded[level] = true;
   return HPCGX_OK;
 }
