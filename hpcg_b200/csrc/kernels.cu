@@ -21,6 +21,7 @@
 //     block to finish sums them in index order and applies the CG scalar
 //     update, so alpha/beta never leave the device.
 #include "kernels.cuh"
+#include "pairs.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -232,9 +233,11 @@ __global__ void k_rank_sum(int nranks, double *const *bufs, int count) {
 // ---------------------------------------------------------------- index checks
 
 // Built with -DHPCGX_CHECKED (libhpcgx_checked.so), the row kernels verify
-// every storage row, vector row and gathered column before using it; a bad
-// one is recorded (the first, as site << 56 | index) and replaced by index 0,
-// which is always inside the buffers, so nothing outside them is touched.
+// every storage row, vector row and gathered column before using it.  The first
+// bad one is recorded (as site << 56 | index).  A bad row is replaced by index 0,
+// which is always inside the buffers and on every vector access's boundary, and
+// a stencil line with a bad column is not read, so nothing outside the buffers
+// is touched.
 // hpcgx_check_status() reports and clears the record.  The stand-in for a
 // memory checker; without the macro the checks compile to nothing.
 #ifdef HPCGX_CHECKED
@@ -444,59 +447,17 @@ __device__ __forceinline__ void stencil_cols(const LevelMat<VT> &A, const RowId 
 
 // ---------------------------------------------------------------- row pairs
 
-// SpMV and the sweeps give a thread the two rows (2i, 2i+1) of an x-line.  On
-// each of the 9 stencil lines (dy, dz) both rows read x[2i-1 .. 2i+2] between
-// them, so a pair gathers 9 x 4 entries with 27 loads (two entries in one
-// vector load) instead of 54, from 9 line addresses instead of 54.
-struct PairId {
-  int64_t row;      // natural index of the even row
-  int64_t ke, ko;   // storage rows
-  int ix, iy, iz;   // of the even row
-  int pos;          // pair inside its line
-  bool left, odd, right;   // x-neighbours of the even row at -1, +1, +2 exist
-  bool ym, yp, zm, zp;     // the lines below / above exist
-};
-
 template <class VT>
 __device__ __forceinline__ PairId pair_of(const LevelMat<VT> &A, const ClassInfo &C, int j0, int t,
                                           int site) {
-  PairId id;
-  const int Le = C.len[0];
-  const int jl = (int)fdiv((uint32_t)t, C.dlen[0]);
-  id.pos = t - jl * Le;
-  const int j = j0 + jl;
-  const int jz = (int)fdiv((uint32_t)j, C.dnyq);
-  id.iy = C.py + 2 * (j - jz * C.nyq);
-  id.iz = C.pz + 2 * jz;
-  id.ix = 2 * id.pos;
-  id.row = ((int64_t)id.iz * A.ny + id.iy) * A.nx + id.ix;
-  id.ke = C.start[0] + (int64_t)j * Le + id.pos;
-  id.ko = C.start[1] + (int64_t)j * C.len[1] + id.pos;
-  id.left = id.pos > 0;
-  id.odd = id.pos < C.len[1];
-  id.right = id.pos + 1 < Le;
-  id.ym = id.iy > 0;
-  id.yp = id.iy + 1 < A.ny;
-  id.zm = id.iz > 0 || A.zlo;
-  id.zp = id.iz + 1 < A.nz || A.zhi;
-  if (!id.odd) id.ko = id.ke;
+  PairId id = pair_at(A, C, j0, t);
 #ifdef HPCGX_CHECKED
-  if (id.row < 0 || id.row + (id.odd ? 1 : 0) >= A.n) {
+  if (!pair_inside(A, id)) {
     check_fail(site, id.row);
-    id.row = 0;
-  }
-  if (id.ke < 0 || id.ke >= A.srows || id.ko < 0 || id.ko >= A.srows) {
-    check_fail(site, id.ke);
-    id.ke = id.ko = 0;
+    redirect(id);
   }
 #endif
   return id;
-}
-
-// Stencil line l = (dz+1)*3 + (dy+1): does it exist for the pair's rows?
-__device__ __forceinline__ bool has_line(const PairId &id, int l) {
-  const int dy = l % 3 - 1, dz = l / 3 - 1;
-  return (dy < 0 ? id.ym : dy > 0 ? id.yp : true) && (dz < 0 ? id.zm : dz > 0 ? id.zp : true);
 }
 
 __device__ __forceinline__ void load2(const double *p, double &u, double &v) {
@@ -522,14 +483,12 @@ __device__ __forceinline__ void store2(float *p, float u, float v) {
 template <class VT, class T>
 __device__ __forceinline__ void load_line(const LevelMat<VT> &A, const PairId &id, const T *xr,
                                           int l, bool on, bool vec, T *v, int site) {
-  const bool ok = on && has_line(id, l);
+  bool ok = on && has_line(id, l);
   const T *q = xr + A.off[3 * l + 1];
 #ifdef HPCGX_CHECKED
-  const int64_t at = id.row + A.off[3 * l + 1];
-  if (ok && ((at - (id.left ? 1 : 0) - A.lo) < 0 ||
-             (at + (id.right ? 2 : id.odd ? 1 : 0) - A.lo) >= A.span)) {
-    check_fail(site, at);
-    q = xr - id.row + 1;
+  if (ok && !line_inside(A, id, vec, l)) {
+    check_fail(site, id.row + A.off[3 * l + 1]);
+    ok = false;
   }
 #endif
   v[0] = v[1] = v[2] = v[3] = T(0);

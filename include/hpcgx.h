@@ -261,7 +261,7 @@ int hpcgx_synchronize(hpcgx_problem *p);
 /* Index-checked build (libhpcgx_checked.so, compiled with -DHPCGX_CHECKED):
  * HPCGX_ECHECK if a kernel has met an out-of-range storage row, vector row
  * or column since the last call (the first one is named in the message; the
- * access itself was redirected into the buffers), else HPCGX_OK.  Synchronises
+ * access itself was redirected into the buffers or left out), else HPCGX_OK.  Synchronises
  * the device.  Always HPCGX_OK in the regular build, which has no checks. */
 int hpcgx_check_status(void);
 

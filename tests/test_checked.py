@@ -1,7 +1,8 @@
 """The index-checked build on the GPU: every kernel family runs on small and
 odd grids, one rank and sharded, and no kernel may meet an out-of-range
 storage row, vector row or column (libhpcgx_checked.so records the first one
-and redirects the access into the buffers; hpcgx_check_status reports it).
+and redirects the access into the buffers or leaves it out;
+hpcgx_check_status reports it; test_pair_index.py checks that answer).
 This stands in for a memory checker, which this GPU pool does not run.
 The checked library is loaded in a child process (HPCGX_LIBRARY=checked is
 read when the library is first loaded)."""
