@@ -165,6 +165,14 @@ struct hpcgx_problem {
   cudaGraphExec_t graph[G_COUNT][2] = {};
   int graph_kernels[G_COUNT] = {};
   int graph_probe[G_COUNT] = {};
+  // the levels with left-out entries when a graph was captured, a bit each: they
+  // pick the form of its kernels
+  int graph_holes[G_COUNT][2] = {};
+  int holed_levels() const {
+    int m = 0;
+    for (int l = 0; l < nlev; ++l) m |= (int)L[l].holes << l;
+    return m;
+  }
   CgMonitor monitor;
   // algorithmic bytes of one iteration of each graph (this implementation's
   // byte model, summed over its launches while the graph is captured)
@@ -277,6 +285,7 @@ struct hpcgx_problem {
       //  pass over colour 6 is served by L2)
       if ((mode & GS_RESTRICT) && c == 0) vec += rows * xb;
       if ((mode & GS_PROLONG) && c == 0) vec += rows * xb;
+      if (A.holes && !mixed) vec += rows * 4.0;   // which entries the row leaves out
       total += nnzb + vec;
     }
     return total;
@@ -463,7 +472,7 @@ struct hpcgx_problem {
         for (int i = 0; i < L[0].nz; ++i) cz += (i + dz >= 0 && i + dz < L[0].nz);
         nnz += cx * cy * cz;
       }
-      spmv_bytes = 8.0 * nnz + 16.0 * n;
+      spmv_bytes = 8.0 * nnz + 16.0 * n + (L[0].holes ? 4.0 * n : 0.0);
     }
     TRY(probed(HPCGX_PROBE_SPMV_FINE, spmv_bytes, [&]() {
       return launch_spmv(L[0], p, Ap, &red, FIN_CG_PAP, st, done, stream);
@@ -478,7 +487,9 @@ struct hpcgx_problem {
 
   int build_graph(int kind, bool timed) {
     cudaGraphExec_t &exec = graph[kind][timed];
-    if (exec && (!timed || graph_probe[kind] == probe)) return HPCGX_OK;
+    const int holed = holed_levels();
+    if (exec && graph_holes[kind][timed] == holed && (!timed || graph_probe[kind] == probe))
+      return HPCGX_OK;
     if (exec) {
       cudaGraphExecDestroy(exec);
       exec = nullptr;
@@ -523,6 +534,7 @@ struct hpcgx_problem {
     cudaGraphDestroy(g);
     CK(e);
     if (timed) graph_probe[kind] = probe;
+    graph_holes[kind][timed] = holed;
     return HPCGX_OK;
   }
 

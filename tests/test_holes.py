@@ -167,3 +167,41 @@ def test_sweeps_keep_to_the_entries(oracle, dims, iz):
     assert sorted(np.flatnonzero(~np.isfinite(want))) == [a, a + 1]
     assert same(P.mg(torch.from_numpy(r).cuda()), want)
     P.close()
+
+
+@pytest.mark.parametrize("times", [False, True], ids=["ahead", "timed"])
+def test_a_solve_follows_the_matrix(oracle, times):
+    """One Problem, loaded with full and with holed matrices in turn: its captured
+    iteration has the kernels of the matrix that is loaded.  iteration_bytes tells
+    them apart: those of a holed level read 4 B per row and launch more."""
+    from hpcg_b200 import Problem
+    from hpcg_b200._lib import CG_MG
+    dims = (16, 8, 8)
+    full, _, _, _ = oracle.hierarchy(*dims, levels=2)
+    n = full[0].nrow
+    some = couplings(full[0])[::5]
+    holed = [edit(full[0], set(some)), full[1]]
+    b = torch.from_numpy(oracle.uniform(3, n, -1.0, 1.0)).cuda()
+
+    def load(p, levels):
+        for l, lev in enumerate(levels):
+            p.load_level(l, lev.nnz, lev.cols, lev.vals)
+        return p
+
+    def solve(p):
+        x = torch.zeros_like(b)
+        out = p.cg(b, x, 50, 1e-10, times=np.zeros(6) if times else None)
+        return out, x, p.iteration_bytes(CG_MG)
+
+    P = Problem(*dims, levels=2)
+    got = [solve(load(P, levels)) for levels in (full, holed, full, holed)]
+    for k in (0, 1):
+        fresh = solve(load(Problem(*dims, levels=2), (full, holed)[k]))
+        for g in got[k::2]:
+            assert g[0] == fresh[0] and torch.equal(g[1], fresh[1]) and g[2] == fresh[2]
+    # two sweeps in which classes 0..2 (a quarter of the rows each) are launched
+    # twice and class 3 once, and the SpMV
+    assert got[1][2] - got[0][2] == 4 * n * (2 * 1.75 + 1)
+    P.generate("hpcg")
+    assert solve(P)[2] == got[0][2]
+    P.close()
