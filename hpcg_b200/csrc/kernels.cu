@@ -935,52 +935,61 @@ k_prolong(int64_t nc, int nxf, int nyf, const T *__restrict__ xc, T *xf,
 // block takes tiles of kTile elements; a thread handles four of a tile, two
 // neighbouring ones and the two half a tile on, with one vector load each, so
 // that a warp's load is one segment and a thread has two loads per vector under
-// way (wide: every vector starts on a two-element boundary).  One element per
-// thread and step before: k_cg_xr at 384^3 331 us -> 270 (5.9 TB/s), a mixed
-// iteration 5.79 -> 5.71 ms; at 64^3 127 -> 123 us.
+// way.  One element per thread and step before: k_cg_xr at 384^3 331 us -> 270
+// (5.9 TB/s), a mixed iteration 5.79 -> 5.71 ms; at 64^3 127 -> 123 us.
+// WIDE: every vector of the launch starts on a two-element boundary; without it a
+// thread takes the same elements one by one, so that a sum's order, and with it
+// its last bits, depend on the length alone and not on where a view starts.
 constexpr int kVec = 4;
 constexpr int kTile = kVec * kThreads;
-template <int N>
+template <int N, bool WIDE>
 struct Width {
   static constexpr int value = N;
 };
 // Runs body(i, width) over [0, n): width 4 for a thread's elements i, i + 1 and
 // i + kTile / 2, i + kTile / 2 + 1 of a tile, width 1 for element i alone.
-template <class F>
-__device__ __forceinline__ void sweep(int64_t n, bool wide, F body) {
-  const int64_t tiles = wide ? n / kTile : 0;
+template <bool WIDE, class F>
+__device__ __forceinline__ void sweep(int64_t n, F body) {
+  const int64_t tiles = n / kTile;
   for (int64_t b = blockIdx.x; b < tiles; b += gridDim.x)
-    body(b * kTile + 2 * (int)threadIdx.x, Width<kVec>());
+    body(b * kTile + 2 * (int)threadIdx.x, Width<kVec, WIDE>());
   for (int64_t i = tiles * kTile + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
-    body(i, Width<1>());
+    body(i, Width<1, WIDE>());
 }
-template <int N, class T>
-__device__ __forceinline__ void get(Width<N>, const T *p, int64_t i, T *v) {
-  if (N == kVec) {
+template <int N, bool WIDE, class T>
+__device__ __forceinline__ void get(Width<N, WIDE>, const T *p, int64_t i, T *v) {
+  if (N == 1) {
+    v[0] = p[i];
+  } else if (WIDE) {
     load2(p + i, v[0], v[1]);
     load2(p + i + kTile / 2, v[2], v[3]);
   } else {
-    v[0] = p[i];
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) v[j] = p[i + (j & 1) + (j >> 1) * (kTile / 2)];
   }
 }
-template <int N, class T>
-__device__ __forceinline__ void put(Width<N>, T *p, int64_t i, const T *v) {
-  if (N == kVec) {
+template <int N, bool WIDE, class T>
+__device__ __forceinline__ void put(Width<N, WIDE>, T *p, int64_t i, const T *v) {
+  if (N == 1) {
+    p[i] = v[0];
+  } else if (WIDE) {
     store2(p + i, v[0], v[1]);
     store2(p + i + kTile / 2, v[2], v[3]);
   } else {
-    p[i] = v[0];
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) p[i + (j & 1) + (j >> 1) * (kTile / 2)] = v[j];
   }
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads)
 k_waxpby(int64_t n, double alpha, const double *x, double beta, const double *y, double *w,
-         int wide, const int *done) {
+         const int *done) {
   if (done && *done) return;
   // The three branches of src/ComputeWAXPBY_ref.cpp:52-67 round differently.
   const int branch = alpha == 1.0 ? 0 : beta == 1.0 ? 1 : 2;
-  sweep(n, wide, [=](int64_t i, auto k) {
+  sweep<WIDE>(n, [=](int64_t i, auto k) {
     double a[kVec], b[kVec];
     get(k, x, i, a);
     get(k, y, i, b);
@@ -993,12 +1002,13 @@ k_waxpby(int64_t n, double alpha, const double *x, double beta, const double *y,
 
 // x.y; the last block stores the total (FIN_STORE into target) or runs a CG
 // scalar step on it (target: the CgState).
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads)
-k_dot(int64_t n, const double *x, const double *y, int wide, Reduce red, int fin, void *target,
+k_dot(int64_t n, const double *x, const double *y, Reduce red, int fin, void *target,
       const int *done) {
   if (done && *done) return;
   double acc = 0.0;
-  sweep(n, wide, [&](int64_t i, auto k) {
+  sweep<WIDE>(n, [&](int64_t i, auto k) {
     double a[kVec], b[kVec];
     get(k, x, i, a);
     get(k, y, i, b);
@@ -1093,16 +1103,15 @@ k_cg_init(int64_t n, const double *__restrict__ b, const double *__restrict__ Ap
 }
 
 // rtz = r.z (src/CG.cpp:109/112); for the flexible solver also z.Ap_{k-1}.
-template <class ZT, bool FLEX>
+template <bool WIDE, class ZT, bool FLEX>
 __global__ void __launch_bounds__(kThreads)
-k_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, int wide, Reduce red,
-        CgState *st) {
+k_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, Reduce red, CgState *st) {
   dependents_launch();
   dependency_wait();
   if (st->done) return;
   const bool two = FLEX && st->k > 1;
   double a0 = 0.0, a1 = 0.0;
-  sweep(n, wide, [&](int64_t i, auto k) {
+  sweep<WIDE>(n, [&](int64_t i, auto k) {
     double a[kVec], b[kVec];
     ZT c[kVec];
     get(k, r, i, a);
@@ -1130,15 +1139,15 @@ k_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, int wide, Red
 // applied here, while p_{k-1} is read anyway, instead of in k_cg_xr: the same
 // operation on the same operands, one read of p fewer per iteration.
 // k_cg_xflush applies the last iteration's update after the loop.
-template <class ZT>
+template <bool WIDE, class ZT>
 __global__ void __launch_bounds__(kThreads)
-k_cg_p(int64_t n, const ZT *z, double *p, int wide, const CgState *st, double *x) {
+k_cg_p(int64_t n, const ZT *z, double *p, const CgState *st, double *x) {
   dependents_launch();
   dependency_wait();
   if (st->done) return;
   const bool first = st->k == 1;
   const double beta = st->beta, alpha = st->alpha;
-  sweep(n, wide, [=](int64_t i, auto k) {
+  sweep<WIDE>(n, [=](int64_t i, auto k) {
     double a[kVec], b[kVec];
     ZT c[kVec];
     get(k, z, i, c);
@@ -1171,15 +1180,16 @@ k_cg_xflush(int64_t n, const double *__restrict__ p, double *x, const CgState *_
 // x += alpha p (unless deferred: x null); r -= alpha Ap; |r|^2
 // (src/CG.cpp:121-124).  r32 (mixed solver): the FP32 copy of r that the
 // V-cycle's finest level reads -- the value it would round r to itself.
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads)
-k_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32, int wide,
+k_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32,
         Reduce red, CgState *st) {
   dependents_launch();
   dependency_wait();
   if (st->done) return;
   const double alpha = st->alpha, malpha = -st->alpha;
   double acc = 0.0;
-  sweep(n, wide, [&](int64_t i, auto k) {
+  sweep<WIDE>(n, [&](int64_t i, auto k) {
     double a[kVec], b[kVec];
     get(k, (const double *)r, i, a);
     get(k, Ap, i, b);
@@ -1882,27 +1892,37 @@ template int launch_gs_class<float, float>(const LevelDev &, int, int, int, cons
                                            float *, const float *, float *, const int *,
                                            cudaStream_t, int, int);
 
-// Two-element access to every vector of a kernel (null: not used).
-template <class... T>
-int all_aligned2(const T *...v) {
-  return (aligned2(v) && ...);
+// Calls go(std::true_type()) if every vector of the launch (null: not used)
+// allows two-element accesses, else go(std::false_type()).
+template <class F, class... T>
+void by_width(F go, const T *...v) {
+  if ((aligned2(v) && ...))
+    go(std::true_type());
+  else
+    go(std::false_type());
 }
 
 int launch_waxpby(int64_t n, double alpha, const double *x, double beta, const double *y,
                   double *w, const int *done, cudaStream_t s) {
-  k_waxpby<<<vector_blocks(n), kThreads, 0, s>>>(n, alpha, x, beta, y, w, all_aligned2(x, y, w), done);
+  by_width([&](auto wide) {
+    k_waxpby<wide.value><<<vector_blocks(n), kThreads, 0, s>>>(n, alpha, x, beta, y, w, done);
+  }, x, y, w);
   return 1;
 }
 
 int launch_dot(int64_t n, const double *x, const double *y, const Reduce &red, double *out,
                cudaStream_t s) {
-  k_dot<<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, all_aligned2(x, y), red, FIN_STORE, out, nullptr);
+  by_width([&](auto wide) {
+    k_dot<wide.value><<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, red, FIN_STORE, out, nullptr);
+  }, x, y);
   return 1;
 }
 
 int launch_dot_finish(int64_t n, const double *x, const double *y, const Reduce &red, int fin,
                       CgState *st, cudaStream_t s) {
-  k_dot<<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, all_aligned2(x, y), red, fin, st, &st->done);
+  by_width([&](auto wide) {
+    k_dot<wide.value><<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, red, fin, st, &st->done);
+  }, x, y);
   return 1;
 }
 
@@ -1949,12 +1969,10 @@ int launch_cg_init(int64_t n, const double *b, const double *Ap, double *r, floa
 template <class ZT>
 int launch_cg_rz(int64_t n, const double *r, const ZT *z, const double *Ap, const Reduce &red,
                  CgState *st, cudaStream_t s) {
-  if (Ap)
-    launch_dependent(k_cg_rz<ZT, true>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap,
-                     all_aligned2(r, z, Ap), red, st);
-  else
-    launch_dependent(k_cg_rz<ZT, false>, dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap,
-                     all_aligned2(r, z, Ap), red, st);
+  by_width([&](auto wide) {
+    launch_dependent(Ap ? k_cg_rz<wide.value, ZT, true> : k_cg_rz<wide.value, ZT, false>,
+                     dim3(vector_blocks(n)), dim3(kThreads), s, n, r, z, Ap, red, st);
+  }, r, z, Ap);
   return 1;
 }
 template int launch_cg_rz<double>(int64_t, const double *, const double *, const double *,
@@ -1964,8 +1982,10 @@ template int launch_cg_rz<float>(int64_t, const double *, const float *, const d
 
 template <class ZT>
 int launch_cg_p(int64_t n, const ZT *z, double *p, CgState *st, cudaStream_t s, double *x) {
-  launch_dependent(k_cg_p<ZT>, dim3(vector_blocks(n)), dim3(kThreads), s, n, z, p,
-                   all_aligned2(z, p, x), st, x);
+  by_width([&](auto wide) {
+    launch_dependent(k_cg_p<wide.value, ZT>, dim3(vector_blocks(n)), dim3(kThreads), s, n, z, p,
+                     (const CgState *)st, x);
+  }, z, p, x);
   return 1;
 }
 template int launch_cg_p<double>(int64_t, const double *, double *, CgState *, cudaStream_t,
@@ -1980,8 +2000,10 @@ int launch_cg_xflush(int64_t n, const double *p, double *x, const CgState *st, c
 
 int launch_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double *r, float *r32,
                  const Reduce &red, CgState *st, cudaStream_t s) {
-  launch_dependent(k_cg_xr, dim3(vector_blocks(n)), dim3(kThreads), s, n, p, Ap, x, r, r32,
-                   all_aligned2(p, Ap, x, r, r32), red, st);
+  by_width([&](auto wide) {
+    launch_dependent(k_cg_xr<wide.value>, dim3(vector_blocks(n)), dim3(kThreads), s, n, p, Ap, x, r,
+                     r32, red, st);
+  }, p, Ap, x, r, r32);
   return 1;
 }
 

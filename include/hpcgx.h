@@ -142,7 +142,8 @@ int hpcgx_mg(hpcgx_problem *p, const double *r, double *x);
 int hpcgx_restriction(hpcgx_problem *p, int level, const double *rf, const double *Axf,
                       double *rc);
 int hpcgx_prolongation(hpcgx_problem *p, int level, const double *xc, double *xf);
-/* ComputeDotProduct (src/ComputeDotProduct.hpp:18); result to host. */
+/* ComputeDotProduct (src/ComputeDotProduct.hpp:18); result to host.  The order of
+ * the sum depends on n alone, so the same data give the same bits. */
 int hpcgx_dot(hpcgx_problem *p, int64_t n, const double *x, const double *y,
               double *result_host);
 /* ComputeWAXPBY (src/ComputeWAXPBY.hpp:18): w = alpha x + beta y. */

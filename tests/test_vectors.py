@@ -1,9 +1,9 @@
 """The vector kernels at the edges of their tiles (1024 elements, four per
-thread) and of the grid (592 and 1184 blocks), with vectors on and off a
-two-element boundary: WAXPBY bit-exact in its three branches
+thread) and of the grid (592 blocks, 1184 above 2^23 elements), with vectors on
+and off a two-element boundary: WAXPBY bit-exact in its three branches
 (src/ComputeWAXPBY_ref.cpp:52-67), in place as well; dot products
 (src/ComputeDotProduct_ref.cpp:48-63) to 1e-13 of the exactly rounded sum of
-products; the residual exact.
+products, the same bits wherever the vectors start; the residual exact.
 """
 import math
 
@@ -13,6 +13,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+# more than 2^23 elements: the larger grid, at its edge and with several tiles a block
+LARGE = [1 << 23, (1 << 23) + 1, 1184 * 1024 * 8 - 1, 1184 * 1024 * 8 + 513]
 SIZES = [1, 2, 255, 1023, 1024, 1025, 2047, 2051, 592 * 1024 - 1, 592 * 1024 + 1, 1184 * 1024 + 513]
 
 
@@ -45,5 +47,36 @@ def test_vectors(P, n, odd):
     assert (z.cpu().numpy() == 0.7 * hx + -1.3 * hy).all()
     want = math.fsum((hx * hy).tolist())
     # each product and the running sums of at most n / 256 terms round once
-    assert abs(P.dot(x, y) - want) <= 1e-13 * np.abs(hx * hy).sum()
+    got = P.dot(x, y)
+    assert abs(got - want) <= 1e-13 * np.abs(hx * hy).sum()
+    # the order of the sum is the length's, not that of where the vectors start
+    assert got == P.dot(x.clone(), y.clone())
     assert P.residual(x, y) == np.abs(hx - hy).max()
+
+
+@pytest.fixture(scope="module")
+def large():
+    from hpcg_b200 import Problem
+    p = Problem(256, 256, 160, levels=1)
+    yield p
+    p.close()
+
+
+@pytest.mark.parametrize("n", LARGE)
+def test_large_vectors(large, n):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, y, w = (torch.empty(n + 2, dtype=torch.float64, device="cuda").uniform_(-1, 1, generator=g)
+               for _ in range(3))
+    hx, hy = x.cpu().numpy(), y.cpu().numpy()
+    # sums of at most n / (1184 * 256) + 1 products a thread, and of the threads'
+    want = float(np.sum(hx[:n].astype(np.longdouble) * hy[1:n + 1]))
+    bound = 1e-13 * float(np.abs(hx[:n] * hy[1:n + 1]).sum())
+    got = large.dot(x[:n], y[1:n + 1])
+    assert abs(got - want) <= bound
+    assert got == large.dot(x[:n], y[1:n + 1].clone())
+    for odd in (0, 1):
+        v, end = w[odd:odd + n], w.clone()
+        large.waxpby(0.7, x[:n], -1.3, y[odd:odd + n], w=v)
+        assert (v.cpu().numpy() == 0.7 * hx[:n] - 1.3 * hy[odd:odd + n]).all()
+        assert torch.equal(w[:odd], end[:odd]) and torch.equal(w[odd + n:], end[odd + n:])
+    assert large.residual(x[:n], y[1:n + 1]) == np.abs(hx[:n] - hy[1:n + 1]).max()
