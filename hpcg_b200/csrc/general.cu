@@ -674,7 +674,7 @@ int general_load_level(GeneralProblem *g, int level, int64_t n, const char *nnz,
   if (level == 0) {
     for (double **v : {&g->r, &g->z, &g->p, &g->Ap, &g->x}) GTRY(g->alloc((void **)v, n * sizeof(double)));
     GTRY(g->alloc((void **)&g->st, sizeof(CgState)));
-    const int64_t blocks = vector_blocks(n);
+    const int64_t blocks = reduce_blocks(n);
     const int64_t cap = 2 * blocks + 2 * ((blocks + 1023) / 1024);
     GTRY(g->alloc((void **)&g->red.partials, cap * sizeof(double)));
     const int64_t counters = 1 + (cap + 1023) / 1024;

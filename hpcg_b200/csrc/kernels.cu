@@ -1610,14 +1610,29 @@ CgMonitor::~CgMonitor() {
   if (slots) cudaFreeHost(slots);
 }
 
-// Blocks of a vector kernel, a tile each at least.  Up to eight per SM to stream
+// Blocks of a tiled vector kernel, a tile each at least.  Up to eight per SM to stream
 // from HBM (25 mixed iterations at 384^3: 5.71 ms each, with four 5.77), four
 // where the vectors stay in L2 and the reduction over the blocks counts (104^3:
 // 237.5 us against 233.7, 128^3: 322 against 317).
-int vector_blocks(int64_t n) {
+static int vector_blocks(int64_t n) {
   const int64_t b = (n + kTile - 1) / kTile;
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * (n > (1 << 23) ? 8 : 4)));
 }
+
+// Blocks of the kernels that take one element per thread and step (k_copy,
+// k_copy_z, k_cg_xflush; with a reduction k_absmax_diff, k_cg_init), four elements
+// a thread at least.  They have a quarter of a tiled kernel's loads under way and
+// want more blocks: eight per SM, k_cg_xflush at 200^3 27.1 us (four: 36.6, twelve:
+// 29.8), k_copy_z 17.3 (18.5, 18.1); at 384^3 198 us (twelve: 215).  A reduction
+// takes as many as still sum in one level (grid_reduce): k_cg_init at 104^3 11.3 us
+// (592 blocks: 12.4, 1099: 13.6), at 200^3 32.0 (38.3, 1184: 34.7), at 384^3 204
+// (1184: 212); k_absmax_diff 9.1 (10.0, 11.5), 25.0 (27.1, 26.8), 132 (132).
+static int element_blocks(int64_t n, bool reduces = false) {
+  const int64_t b = (n + 4 * kThreads - 1) / (4 * kThreads);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(b, reduces ? kReduceGroup : 148 * 8));
+}
+
+int reduce_blocks(int64_t n) { return std::max(vector_blocks(n), element_blocks(n, true)); }
 
 void plan_level(LevelDev &L, int nx, int ny, int nz) {
   L.nx = nx;
@@ -1928,7 +1943,7 @@ int launch_dot_finish(int64_t n, const double *x, const double *y, const Reduce 
 
 int launch_absmax_diff(int64_t n, const double *a, const double *b, const Reduce &red,
                        double *out, cudaStream_t s) {
-  k_absmax_diff<<<vector_blocks(n), kThreads, 0, s>>>(n, a, b, red, out);
+  k_absmax_diff<<<element_blocks(n, true), kThreads, 0, s>>>(n, a, b, red, out);
   return 1;
 }
 
@@ -1945,7 +1960,7 @@ int launch_prolongation(int64_t nc, const LevelDev &F, const double *xc, double 
 }
 
 int launch_copy(int64_t n, const double *x, double *y, const int *done, cudaStream_t s) {
-  k_copy<<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, done);
+  k_copy<<<element_blocks(n), kThreads, 0, s>>>(n, x, y, done);
   return 1;
 }
 
@@ -1962,7 +1977,7 @@ int launch_fill_normal(int64_t n, uint64_t seed, uint64_t offset, double *v, cud
 
 int launch_cg_init(int64_t n, const double *b, const double *Ap, double *r, float *r32,
                    const Reduce &red, CgState *st, cudaStream_t s) {
-  k_cg_init<<<vector_blocks(n), kThreads, 0, s>>>(n, b, Ap, r, r32, red, st);
+  k_cg_init<<<element_blocks(n, true), kThreads, 0, s>>>(n, b, Ap, r, r32, red, st);
   return 1;
 }
 
@@ -1994,7 +2009,7 @@ template int launch_cg_p<float>(int64_t, const float *, double *, CgState *, cud
                                 double *);
 
 int launch_cg_xflush(int64_t n, const double *p, double *x, const CgState *st, cudaStream_t s) {
-  k_cg_xflush<<<vector_blocks(n), kThreads, 0, s>>>(n, p, x, st);
+  k_cg_xflush<<<element_blocks(n), kThreads, 0, s>>>(n, p, x, st);
   return 1;
 }
 
@@ -2008,7 +2023,7 @@ int launch_cg_xr(int64_t n, const double *p, const double *Ap, double *x, double
 }
 
 int launch_copy_z(int64_t n, const double *r, double *z, const CgState *st, cudaStream_t s) {
-  k_copy_z<<<vector_blocks(n), kThreads, 0, s>>>(n, r, z, st);
+  k_copy_z<<<element_blocks(n), kThreads, 0, s>>>(n, r, z, st);
   return 1;
 }
 

@@ -192,6 +192,8 @@ int launch_adjoint_grad(const LevelDev &L, const double *lambda, const double *x
                          cudaStream_t s);
 
 // Reduction helpers -------------------------------------------------------
-int vector_blocks(int64_t n);
+// The most blocks of a reduction over n elements (its scratch; never fewer for a
+// larger n).
+int reduce_blocks(int64_t n);
 
 }  // namespace hpcgx

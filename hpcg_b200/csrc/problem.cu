@@ -1608,7 +1608,7 @@ int hpcgx_create_slab(int device, int nx, int ny, int nz, int levels, int nranks
     red_cap = std::max<int64_t>(red_cap, red_need(A.spmv_blocks));
   }
   const int64_t n = p->L[0].n;
-  red_cap = std::max<int64_t>(red_cap, red_need(vector_blocks(n)));
+  red_cap = std::max<int64_t>(red_cap, red_need(reduce_blocks(n)));
   const int64_t plane0 = (int64_t)p->L[0].nx * p->L[0].ny;
   for (double **v : {&p->b, &p->x, &p->r, &p->Ap, &p->tmp})
     if ((rc = p->alloc((void **)v, n * sizeof(double)))) return bail(rc);
@@ -1671,7 +1671,7 @@ int hpcgx_load_level_general(hpcgx_problem *p, int level, int64_t nrows, const c
     for (double **v : {&p->b, &p->x})
       TRY(p->alloc((void **)v, nrows * sizeof(double)));
     TRY(p->alloc((void **)&p->result, 4 * sizeof(double)));
-    const int64_t blocks = vector_blocks(nrows);
+    const int64_t blocks = reduce_blocks(nrows);
     const int64_t cap = 2 * blocks + 2 * ((blocks + 1023) / 1024);
     TRY(p->alloc((void **)&p->red.partials, cap * sizeof(double)));
     const int64_t counters = 1 + (cap + 1023) / 1024;

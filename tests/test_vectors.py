@@ -1,6 +1,6 @@
 """The vector kernels at the edges of their tiles (1024 elements, four per
-thread) and of the grid (592 blocks, 1184 above 2^23 elements), with vectors on
-and off a two-element boundary: WAXPBY bit-exact in its three branches
+thread) and of the grid (592 blocks, 1184 above 2^23 elements; 1024 for the
+residual), with vectors on and off a two-element boundary: WAXPBY bit-exact in its three branches
 (src/ComputeWAXPBY_ref.cpp:52-67), in place as well; dot products
 (src/ComputeDotProduct_ref.cpp:48-63) to 1e-13 of the exactly rounded sum of
 products, the same bits wherever the vectors start; the residual exact.
@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 
 # more than 2^23 elements: the larger grid, at its edge and with several tiles a block
 LARGE = [1 << 23, (1 << 23) + 1, 1184 * 1024 * 8 - 1, 1184 * 1024 * 8 + 513]
-SIZES = [1, 2, 255, 1023, 1024, 1025, 2047, 2051, 592 * 1024 - 1, 592 * 1024 + 1, 1184 * 1024 + 513]
+SIZES = [1, 2, 255, 1023, 1024, 1025, 2047, 2051, 592 * 1024 - 1, 592 * 1024 + 1,
+         1024 * 1024 - 1, 1024 * 1024 + 1, 1184 * 1024 + 513]
 
 
 @pytest.fixture(scope="module")
