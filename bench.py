@@ -731,7 +731,7 @@ def main():
                                          "vectors) / time: work this design does not do, so it "
                                          "exceeds the HBM peak; for comparison with other HPCG "
                                          "implementations only"},
-        "roofline": roofline(PROBE_SPMV_FINE, "k_spmv<double,double,1,0>"),
+        "roofline": roofline(PROBE_SPMV_FINE, "k_spmv<double,double,2,0>"),
         "roofline_gs_bwd": roofline(PROBE_GS_FINE_BWD, "k_gs_class<0,1,-1,3,0,bf16,f32,f32>"),
         "roofline_gs_fine_all_modes": roofline(PROBE_GS_FINE, "k_gs_class finest level, all modes"),
         "e2e": {"value": t_e2e, "unit": "s", "h2d_bytes_per_step": world * 2 * n * 8,

@@ -269,6 +269,7 @@ __device__ __forceinline__ int64_t check_index(int64_t i, int64_t n, int site) {
 struct ClassSet {
   ClassInfo c[4];
   int nblk[4];     // blocks of each class
+  int turns;       // groups of 256 pairs a block takes
   int common;      // min over the classes of nblk
   int total;       // sum of nblk: the grid
 };
@@ -517,15 +518,19 @@ __device__ __forceinline__ T term_sub(uint32_t out, int s, T sum, T v, T x) {
 
 // y = A x, rows summed left to right over the slots as ComputeSPMV_ref does
 // (src/ComputeSPMV_ref.cpp:64-70).  With DOT, also reduces sum_i x_i y_i (the
-// p.Ap of CG, src/CG.cpp:119) and runs the finishing scalar step.  A block
-// takes 256 consecutive pairs of one class, whatever lines they lie on (rows
-// have no order to keep), so no thread idles on ragged lines; the classes are
-// interleaved block by block (class_block).  HBM bounds it: 8 B per nonzero and
-// 16 B per row at 256^3 is 3.86 GB, 568 us = 6.8 TB/s, 1.04 of the measured
-// copy rate (one row per thread and stored int32 columns: 824 us; 104^3: 59
-// against 78 us).  FP64 holds a z-plane's 18 values and 12 entries per step
-// (128 registers, two blocks per SM); one and three blocks measured the same.
-template <class VT, class T, bool DOT, bool GEN>
+// p.Ap of CG, src/CG.cpp:119) and runs the finishing scalar step (DOT_FUSED) or
+// leaves a partial sum per block for k_sum_partials (DOT_PARTS, see
+// kDotLaunchRows).  A block takes 256 consecutive pairs of one class (DOT_PARTS:
+// cs.turns times as many), whatever lines they lie on (rows have no order to
+// keep), so no thread idles on ragged lines; the classes are interleaved block by
+// block (class_block).  HBM bounds it: 8 B per nonzero and 16 B per row at 256^3
+// is 3.86 GB, 568 us = 6.8 TB/s, 1.04 of the measured copy rate (one row per
+// thread and stored int32 columns: 824 us, and with derived columns, as the mixed
+// solver had it: 596; 104^3: 59 against 78 us).  FP64 holds a z-plane's 18 values
+// and 12 entries per step (128 registers, two blocks per SM); one and three blocks
+// measured the same.
+enum SpmvDot { DOT_NONE = 0, DOT_FUSED = 1, DOT_PARTS = 2 };
+template <class VT, class T, int DOT, bool GEN>
 __global__ void __launch_bounds__(kThreads, std::is_same<VT, double>::value ? 2 : 4)
 k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet cs, const T *x,
        T *y, int wide, Reduce red, int fin, void *fin_target, const int *done) {
@@ -534,61 +539,95 @@ k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet 
   int q, b;
   class_block(cs, (int)blockIdx.x, q, b);
   const ClassInfo &C = cs.c[q];
-  const int t = b * kThreads + (int)threadIdx.x;
   double acc = 0.0;
-  const bool act = t < C.lines * C.len[0];
-  PairId id;
-  T ve[9], vo[9];
-  uint32_t oe = 0u, oo = 0u;   // left-out entries of the two rows
-  if (act) {
-    id = pair_of(A, C, 0, t, 1);
-    if (GEN && A.left_out) {
-      oe = A.left_out[id.ke];
-      oo = A.left_out[id.ko];
+  const int turns = DOT == DOT_PARTS ? cs.turns : 1;
+#pragma unroll 1
+  for (int turn = 0; turn < turns; ++turn) {
+    const int t = (b * turns + turn) * kThreads + (int)threadIdx.x;
+    const bool act = t < C.lines * C.len[0];
+    PairId id;
+    T ve[9], vo[9];
+    uint32_t oe = 0u, oo = 0u;   // left-out entries of the two rows
+    if (act) {
+      id = pair_of(A, C, 0, t, 1);
+      if (GEN && A.left_out) {
+        oe = A.left_out[id.ke];
+        oo = A.left_out[id.ko];
+      }
+      load_vals(A.vals, id.ke, 0, NeedAll(), ve);
+      load_vals(A.vals, id.ko, 0, NeedAll(), vo);
     }
-    load_vals(A.vals, id.ke, 0, NeedAll(), ve);
-    load_vals(A.vals, id.ko, 0, NeedAll(), vo);
+    if (turn == 0) {
+      dependency_wait();
+      if (done && *done) return;
+    }
+    if (act) {
+      const T *xr = x + id.row;
+      T se = T(0), so = T(0), xe = T(0), xo = T(0);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        T v[3][4];
+        if (p > 0) {
+          load_vals(A.vals, id.ke, p, NeedAll(), ve);
+          load_vals(A.vals, id.ko, p, NeedAll(), vo);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) load_line(A, id, xr, 3 * p + i, true, vec, v[i], 2);
+#pragma unroll
+        for (int s = 0; s < 9; ++s) {
+          se = term_add(oe, 9 * p + s, se, ve[s], v[s / 3][s % 3]);
+          so = term_add(oo, 9 * p + s, so, vo[s], v[s / 3][s % 3 + 1]);
+        }
+        if (p == 1) {
+          xe = v[1][1];
+          xo = v[1][2];
+        }
+      }
+      if (vec && id.odd) {
+        store2(y + id.row, se, so);
+      } else {
+        y[id.row] = se;
+        if (id.odd) y[id.row + 1] = so;
+      }
+      if (DOT) {
+        acc += (double)xe * (double)se;
+        if (id.odd) acc += (double)xo * (double)so;
+      }
+    }
   }
-  dependency_wait();
-  if (done && *done) return;
-  if (act) {
-    const T *xr = x + id.row;
-    T se = T(0), so = T(0), xe = T(0), xo = T(0);
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      T v[3][4];
-      if (p > 0) {
-        load_vals(A.vals, id.ke, p, NeedAll(), ve);
-        load_vals(A.vals, id.ko, p, NeedAll(), vo);
-      }
-#pragma unroll
-      for (int i = 0; i < 3; ++i) load_line(A, id, xr, 3 * p + i, true, vec, v[i], 2);
-#pragma unroll
-      for (int s = 0; s < 9; ++s) {
-        se = term_add(oe, 9 * p + s, se, ve[s], v[s / 3][s % 3]);
-        so = term_add(oo, 9 * p + s, so, vo[s], v[s / 3][s % 3 + 1]);
-      }
-      if (p == 1) {
-        xe = v[1][1];
-        xo = v[1][2];
-      }
-    }
-    if (vec && id.odd) {
-      store2(y + id.row, se, so);
-    } else {
-      y[id.row] = se;
-      if (id.odd) y[id.row + 1] = so;
-    }
-    if (DOT) {
-      acc = (double)xe * (double)se;
-      if (id.odd) acc += (double)xo * (double)so;
-    }
-  }
-  if (DOT) {
+  if (DOT == DOT_FUSED) {
     double v[1] = {acc}, tot[1];
     if (grid_reduce<1>(v, red, tot) && threadIdx.x == 0)
       finish_or_defer<1>(red, fin, fin_target, tot);
   }
+  if (DOT == DOT_PARTS) {
+    __shared__ double sh[kThreads / 32];
+    const double w = warp_red<false>(acc);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = w;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double sum = 0.0;
+      for (int i = 0; i < kThreads / 32; ++i) sum += sh[i];
+      red.partials[blockIdx.x] = sum;
+    }
+  }
+}
+
+// The sum of the n partials p of a launch with DOT_PARTS, kReduceGroup of them a
+// block, and its scalar step.
+__global__ void __launch_bounds__(kThreads)
+k_sum_partials(const double *p, int64_t n, Reduce red, int fin, void *target, const int *done) {
+  dependents_launch();
+  dependency_wait();
+  if (done && *done) return;
+  double acc = 0.0;
+#pragma unroll
+  for (int j = 0; j < kReduceGroup / kThreads; ++j) {
+    const int64_t i = blockIdx.x * (int64_t)kReduceGroup + j * kThreads + threadIdx.x;
+    if (i < n) acc += p[i];
+  }
+  double v[1] = {acc}, tot[1];
+  if (grid_reduce<1>(v, red, tot) && threadIdx.x == 0) finish_or_defer<1>(red, fin, target, tot);
 }
 
 // ---------------------------------------------------------------- Gauss-Seidel
@@ -1573,16 +1612,17 @@ bool aligned2(const T *v) {
   return reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0;
 }
 
-// The SpMV's blocks: 256 consecutive pairs of a class each.
-ClassSet classes_of(const LevelDev &L) {
+// The SpMV's blocks: `turns` groups of 256 consecutive pairs of a class each.
+ClassSet classes_of(const LevelDev &L, int turns = 1) {
   ClassSet cs;
+  cs.turns = turns;
   cs.common = INT_MAX;
   cs.total = 0;
   for (int q = 0; q < 4; ++q) {
     const ClassInfo &C = L.cls[q];
     const int64_t pairs = (int64_t)C.lines * C.len[0];
     cs.c[q] = C;
-    cs.nblk[q] = (int)((pairs + kThreads - 1) / kThreads);
+    cs.nblk[q] = (int)((pairs + turns * kThreads - 1) / (turns * kThreads));
     cs.common = std::min(cs.common, cs.nblk[q]);
     cs.total += cs.nblk[q];
   }
@@ -1719,21 +1759,40 @@ int launch_get_diagonal(const LevelDev &L, double *diag, cudaStream_t s) {
   return 1;
 }
 
+// Rows from which the SpMV's dot product is summed by a launch of its own, after
+// blocks of two turns.  With it fused each block ends in a fence and a counter,
+// 0.3 us that keep its place on the SM: at 512^3, with 262,144 blocks of 5 us,
+// p.Ap takes 4894 us fused and 4695 so (one row per thread and half the blocks,
+// before the pairs: 4735), at 448^3 3216 and 3120, at 384^3 1979 and 1942, at 352^3
+// 1509 and 1499; at 256^3 585 both, and below that the launch costs what it saves.
+// (512^3 and 384^3 on another device, fused 4815 and 1944: so 4600 and 1920; one turn
+// and a launch 4689 and 1939; two or four turns, fused, 4763 and 1988, 4652 and 1962.)
+constexpr int64_t kDotLaunchRows = 1 << 25;
+
 int launch_spmv(const LevelDev &L, const double *x, double *y, const Reduce *dot, int fin,
                 void *fin_target, const int *done, cudaStream_t s) {
   if (L.spmv_blocks == 0) return 0;
-  const ClassSet cs = classes_of(L);
-  const LevelMat<double> A = mat_of(L, L.vals);
   const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(y);
+  const bool gen = !vec || L.holes;
+  const LevelMat<double> A = mat_of(L, L.vals);
   const Reduce red = dot ? *dot : Reduce();
+  const bool parts = dot && L.n >= kDotLaunchRows;
+  const ClassSet cs = classes_of(L, parts ? 2 : 1);
   auto go = [&](auto kernel) {
     launch_dependent(kernel, dim3(cs.total), dim3(kThreads), s, A, cs, x, y, vec, red, fin,
                      fin_target, done);
     return 1;
   };
-  if (vec && !L.holes)
-    return dot ? go(k_spmv<double, double, true, false>) : go(k_spmv<double, double, false, false>);
-  return dot ? go(k_spmv<double, double, true, true>) : go(k_spmv<double, double, false, true>);
+  if (!dot)
+    return gen ? go(k_spmv<double, double, DOT_NONE, true>) : go(k_spmv<double, double, DOT_NONE, false>);
+  if (!parts)
+    return gen ? go(k_spmv<double, double, DOT_FUSED, true>) : go(k_spmv<double, double, DOT_FUSED, false>);
+  gen ? go(k_spmv<double, double, DOT_PARTS, true>) : go(k_spmv<double, double, DOT_PARTS, false>);
+  Reduce sums = red;   // the partials' own scratch follows them (reduce_scratch)
+  sums.partials = red.partials + cs.total;
+  launch_dependent(k_sum_partials, dim3((cs.total + kReduceGroup - 1) / kReduceGroup), dim3(kThreads),
+                   s, (const double *)red.partials, (int64_t)cs.total, sums, fin, fin_target, done);
+  return 2;
 }
 
 int launch_spmv32(const LevelDev &L, const float *x, float *y, cudaStream_t s) {
@@ -1745,7 +1804,7 @@ int launch_spmv32(const LevelDev &L, const float *x, float *y, cudaStream_t s) {
                      Reduce(), 0, (void *)nullptr, (const int *)nullptr);
     return 1;
   };
-  return vec ? go(k_spmv<uint16_t, float, false, false>) : go(k_spmv<uint16_t, float, false, true>);
+  return vec ? go(k_spmv<uint16_t, float, DOT_NONE, false>) : go(k_spmv<uint16_t, float, DOT_NONE, true>);
 }
 
 template <class T>
