@@ -278,6 +278,8 @@ struct hpcgx_problem {
         const int dx = s % 3 - 1, dy = (s / 3) % 3 - 1, dz = s / 9 - 1;
         const int64_t cnt = axis_count(A.nx, px, dx) * axis_count(A.ny, py, dy) *
                             axis_count(A.nz, pz, dz);
+        // a zero-guess launch has no term of a higher colour
+        if (mode == GS_ZERO_GUESS && s != HPCGX_DIAG_SLOT && (c ^ slot_mask(s)) > c) continue;
         nnzb += (double)cnt * vb;
       }
       double vec = rows * (rb + xb + ((mode & GS_ZERO_GUESS) ? 0.0 : xb));
