@@ -529,13 +529,23 @@ __device__ __forceinline__ T term_sub(uint32_t out, int s, T sum, T v, T x) {
 // solver had it: 596; 104^3: 59 against 78 us).  FP64 holds a z-plane's 18 values
 // and 12 entries per step (128 registers, two blocks per SM); one and three blocks
 // measured the same.
+// The forms of the row-pair kernels.  FORM_WIDE: every vector starts on a
+// two-element boundary and lines are even, so that two entries go with one
+// access.  FORM_SCALAR: neither is sure.  FORM_HOLES: a matrix with left-out
+// entries (LevelMat::left_out), vectors of either kind.
+enum Form { FORM_WIDE = 0, FORM_SCALAR = 1, FORM_HOLES = 2 };
+template <int FORM>
+__device__ __forceinline__ bool is_wide(int vec) {
+  return FORM == FORM_WIDE || (FORM == FORM_HOLES && vec);
+}
+
 enum SpmvDot { DOT_NONE = 0, DOT_FUSED = 1, DOT_PARTS = 2 };
-template <class VT, class T, int DOT, bool GEN>
+template <class VT, class T, int DOT, int FORM>
 __global__ void __launch_bounds__(kThreads, std::is_same<VT, double>::value ? 2 : 4)
 k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet cs, const T *x,
        T *y, int wide, Reduce red, int fin, void *fin_target, const int *done) {
   dependents_launch();
-  const bool vec = !GEN || wide;
+  const bool vec = is_wide<FORM>(wide);
   int q, b;
   class_block(cs, (int)blockIdx.x, q, b);
   const ClassInfo &C = cs.c[q];
@@ -550,7 +560,7 @@ k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet 
     uint32_t oe = 0u, oo = 0u;   // left-out entries of the two rows
     if (act) {
       id = pair_of(A, C, 0, t, 1);
-      if (GEN && A.left_out) {
+      if (FORM == FORM_HOLES && A.left_out) {
         oe = A.left_out[id.ke];
         oo = A.left_out[id.ko];
       }
@@ -701,7 +711,7 @@ __device__ __forceinline__ T gs_tail(uint32_t out, int c, const V &val, const T 
 // to left forward and from left to right backward: a chunk then finds the
 // neighbours that its first row must see unchanged unchanged, and those that
 // its second row must see updated updated.
-template <int DIR, bool ZERO, bool SYM3, bool AHEAD, class VT, class T, class RT>
+template <int DIR, bool ZERO, bool SYM3, bool AHEAD, int FORM, class VT, class T, class RT>
 __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo &C, int ce, int j0,
                                          int j1, bool zero, bool pro, bool res, bool vec,
                                          const uint32_t *left_out, const RT *r, T *x, const T *xc,
@@ -718,7 +728,7 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
     const int t = (DIR == 0 ? chunks - 1 - ch : ch) * nb + tid;
     const bool act = t < cnt;
     PairId id;
-    RowVals<VT> ve, vo;
+    RowVals<VT> ve, vo{};
     uint32_t oe = 0u, oo = 0u;
     T xl[5][4];
     T se = T(0), so = T(0), ax = T(0), xe = T(0), xo = T(0), re = T(0);
@@ -736,7 +746,7 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
 #pragma unroll
       for (int p = 0; p < 3; ++p) {
         ve.load(A.vals, id.ke, p, need_e);
-        vo.load(A.vals, id.ko, p, need_o);
+        if (FORM == FORM_WIDE || id.odd) vo.load(A.vals, id.ko, p, need_o);
       }
     }
     if (AHEAD && ch == 0) {
@@ -880,11 +890,14 @@ __device__ __forceinline__ void prefetch_lines(const LevelMat<VT> &A, const Clas
 // sharded sweep splits its first launch into the lines that read no halo plane
 // and the rest).  Q >= 0 fixes the class at compile time, which lets the
 // zero-guess sweep drop the loads of the skipped slots.
-// GEN: the general form, for vectors without two-element alignment and matrices
-// with left-out entries; the other form has neither test in it.
+// FORM: see Form.  Each form holds its own tests only, and the last pair of an odd
+// line no values of a second row: one form for everything but FORM_WIDE, with a
+// test for left-out entries at every term, took 1475 us for the symmetric FP64
+// sweep at 255^3 (1190 so; with one row per thread 1601) and 640 for the BF16 one
+// (460; 512), 6849 from vectors off the boundary at 384^3 (5380 before the pairs).
 // Against one row per thread with a second load phase for the second colour
 // (before) the pair issues all its loads once: FP64, HBM-bound, the symmetric
-// sweep at 256^3 takes 1186 us = 6.4 TB/s of 8 B per nonzero and pass (before,
+// sweep at 256^3 takes 1186 us = 6.1 TB/s of 8 B per nonzero and pass (before,
 // with stored columns: 1596 us), the V-cycle at 104^3, latency-bound on its
 // coarse levels, 399 us (545).  BF16: 2 B per nonzero leaves the loads' latency
 // and x, which every class launch gathers again, as the bound: V-cycle at
@@ -895,7 +908,7 @@ __device__ __forceinline__ void prefetch_lines(const LevelMat<VT> &A, const Clas
 // BF16 at 64^3 136 us (218), at 256^3 937 us (1137), at 384^3 2934 us (3293).
 // The BF16 kernels with three blocks per SM wait first (AHEAD off): values held
 // over the wait cost them spills (384^3: 3353 us).
-template <int MODE, int DIR, int Q, int MINB, bool GEN, class VT, class T, class RT>
+template <int MODE, int DIR, int Q, int MINB, int FORM, class VT, class T, class RT>
 __global__ void __launch_bounds__(kThreads, MINB)
 k_gs_class(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassInfo C, int lpb,
            int jbeg, int jend, int vec, const RT *r, T *x, const T *xc, T *rc, const int *done) {
@@ -909,9 +922,10 @@ k_gs_class(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ Class
     const int jn = j0 + kAhead * lpb;
     if (jn < jend) prefetch_lines(A, C, jn, min(jn + lpb, jend));
   }
-  gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0, MINB != 3>(
+  gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0, MINB != 3, FORM>(
       A, C, 2 * (Q >= 0 ? Q : C.q), j0, min(j0 + lpb, jend), false, (MODE & GS_PROLONG) != 0,
-      (MODE & GS_RESTRICT) != 0, !GEN || vec, GEN ? A.left_out : nullptr, r, x, xc, rc, sh, done);
+      (MODE & GS_RESTRICT) != 0, is_wide<FORM>(vec), FORM == FORM_HOLES ? A.left_out : nullptr, r, x,
+      xc, rc, sh, done);
 }
 
 // Residual restricted at the injected points (colour 0: even ix, iy, iz):
@@ -1773,7 +1787,6 @@ int launch_spmv(const LevelDev &L, const double *x, double *y, const Reduce *dot
                 void *fin_target, const int *done, cudaStream_t s) {
   if (L.spmv_blocks == 0) return 0;
   const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(y);
-  const bool gen = !vec || L.holes;
   const LevelMat<double> A = mat_of(L, L.vals);
   const Reduce red = dot ? *dot : Reduce();
   const bool parts = dot && L.n >= kDotLaunchRows;
@@ -1783,11 +1796,15 @@ int launch_spmv(const LevelDev &L, const double *x, double *y, const Reduce *dot
                      fin_target, done);
     return 1;
   };
-  if (!dot)
-    return gen ? go(k_spmv<double, double, DOT_NONE, true>) : go(k_spmv<double, double, DOT_NONE, false>);
-  if (!parts)
-    return gen ? go(k_spmv<double, double, DOT_FUSED, true>) : go(k_spmv<double, double, DOT_FUSED, false>);
-  gen ? go(k_spmv<double, double, DOT_PARTS, true>) : go(k_spmv<double, double, DOT_PARTS, false>);
+  auto form = [&](auto dot_kind) {
+    constexpr int D = decltype(dot_kind)::value;
+    return L.holes ? go(k_spmv<double, double, D, FORM_HOLES>)
+           : vec   ? go(k_spmv<double, double, D, FORM_WIDE>)
+                   : go(k_spmv<double, double, D, FORM_SCALAR>);
+  };
+  if (!dot) return form(std::integral_constant<int, DOT_NONE>());
+  if (!parts) return form(std::integral_constant<int, DOT_FUSED>());
+  form(std::integral_constant<int, DOT_PARTS>());
   Reduce sums = red;   // the partials' own scratch follows them (reduce_scratch)
   sums.partials = red.partials + cs.total;
   launch_dependent(k_sum_partials, dim3((cs.total + kReduceGroup - 1) / kReduceGroup), dim3(kThreads),
@@ -1804,7 +1821,8 @@ int launch_spmv32(const LevelDev &L, const float *x, float *y, cudaStream_t s) {
                      Reduce(), 0, (void *)nullptr, (const int *)nullptr);
     return 1;
   };
-  return vec ? go(k_spmv<uint16_t, float, DOT_NONE, false>) : go(k_spmv<uint16_t, float, DOT_NONE, true>);
+  return vec ? go(k_spmv<uint16_t, float, DOT_NONE, FORM_WIDE>)
+             : go(k_spmv<uint16_t, float, DOT_NONE, FORM_SCALAR>);
 }
 
 template <class T>
@@ -1848,7 +1866,7 @@ GsBlock gs_block(const ClassInfo &C) {
 }
 
 // The class kernels, by blocks per SM and form (k_gs_class).
-template <int MINB, bool GEN, class T, class RT>
+template <int MINB, int FORM, class T, class RT>
 int launch_gs_rows(const LevelDev &L, int q, int backward, int mode, const RT *r, T *x,
                    const T *xc, T *rc, const int *done, cudaStream_t s, int jbeg, int jend,
                    GsBlock gb, int vec) {
@@ -1860,24 +1878,24 @@ int launch_gs_rows(const LevelDev &L, int q, int backward, int mode, const RT *r
     launch_dependent(kernel, g, b, s, A, C, gb.lines, jbeg, jend, vec, r, x, xc, rc, done);
     return 1;
   };
-  if (mode == GS_SYM3 && q == 3) return go(k_gs_class<GS_SYM3, 0, 3, MINB, GEN, VT, T, RT>);
+  if (mode == GS_SYM3 && q == 3) return go(k_gs_class<GS_SYM3, 0, 3, MINB, FORM, VT, T, RT>);
   if (mode == (GS_SYM3 | GS_ZERO_GUESS) && q == 3)
-    return go(k_gs_class<GS_SYM3 | GS_ZERO_GUESS, 0, 3, MINB, GEN, VT, T, RT>);
+    return go(k_gs_class<GS_SYM3 | GS_ZERO_GUESS, 0, 3, MINB, FORM, VT, T, RT>);
   if (mode == GS_ZERO_GUESS && !backward) {
     switch (q) {
-      case 0: return go(k_gs_class<GS_ZERO_GUESS, 0, 0, MINB, GEN, VT, T, RT>);
-      case 1: return go(k_gs_class<GS_ZERO_GUESS, 0, 1, MINB, GEN, VT, T, RT>);
-      case 2: return go(k_gs_class<GS_ZERO_GUESS, 0, 2, MINB, GEN, VT, T, RT>);
-      default: return go(k_gs_class<GS_ZERO_GUESS, 0, 3, MINB, GEN, VT, T, RT>);
+      case 0: return go(k_gs_class<GS_ZERO_GUESS, 0, 0, MINB, FORM, VT, T, RT>);
+      case 1: return go(k_gs_class<GS_ZERO_GUESS, 0, 1, MINB, FORM, VT, T, RT>);
+      case 2: return go(k_gs_class<GS_ZERO_GUESS, 0, 2, MINB, FORM, VT, T, RT>);
+      default: return go(k_gs_class<GS_ZERO_GUESS, 0, 3, MINB, FORM, VT, T, RT>);
     }
   }
   if (mode == GS_RESTRICT && backward && q == 0)
-    return go(k_gs_class<GS_RESTRICT, 1, 0, MINB, GEN, VT, T, RT>);
+    return go(k_gs_class<GS_RESTRICT, 1, 0, MINB, FORM, VT, T, RT>);
   if (mode == GS_PROLONG && !backward && q == 0)
-    return go(k_gs_class<GS_PROLONG, 0, 0, MINB, GEN, VT, T, RT>);
+    return go(k_gs_class<GS_PROLONG, 0, 0, MINB, FORM, VT, T, RT>);
   if (mode != GS_PLAIN) return 0;
-  return backward ? go(k_gs_class<GS_PLAIN, 1, -1, MINB, GEN, VT, T, RT>)
-                  : go(k_gs_class<GS_PLAIN, 0, -1, MINB, GEN, VT, T, RT>);
+  return backward ? go(k_gs_class<GS_PLAIN, 1, -1, MINB, FORM, VT, T, RT>)
+                  : go(k_gs_class<GS_PLAIN, 0, -1, MINB, FORM, VT, T, RT>);
 }
 
 template <class T, class RT>
@@ -1889,14 +1907,23 @@ int launch_gs_class(const LevelDev &L, int q, int backward, int mode, const RT *
   const GsBlock gb = gs_block<T>(L.cls[q]);
   const int vec = L.nx % 2 == 0 && aligned2(x) && aligned2(r);
   constexpr bool fp64 = std::is_same<T, double>::value;
-  if (!vec || (fp64 && L.holes))
-    return launch_gs_rows<fp64 ? 1 : 2, true>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg,
-                                              jend, gb, vec);
-  if (!fp64 && (int64_t)L.cls[q].lines * L.cls[q].len[0] > kManyPairs)
-    return launch_gs_rows<fp64 ? 1 : 3, false>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg,
-                                               jend, gb, vec);
-  return launch_gs_rows<fp64 ? 1 : 2, false>(L, q, backward, mode, r, x, xc, rc, done, s, jbeg,
-                                             jend, gb, vec);
+  const bool many = (int64_t)L.cls[q].lines * L.cls[q].len[0] > kManyPairs;
+  auto rows = [&](auto minb, auto form) {
+    return launch_gs_rows<decltype(minb)::value, decltype(form)::value>(L, q, backward, mode, r, x, xc, rc,
+                                                                        done, s, jbeg, jend, gb, vec);
+  };
+  using std::integral_constant;
+  constexpr integral_constant<int, FORM_WIDE> wide{};
+  constexpr integral_constant<int, FORM_SCALAR> scalar{};
+  if constexpr (fp64) {
+    constexpr integral_constant<int, 1> one{};
+    return L.holes ? rows(one, integral_constant<int, FORM_HOLES>()) : vec ? rows(one, wide) : rows(one, scalar);
+  } else {
+    constexpr integral_constant<int, 2> two{};
+    constexpr integral_constant<int, 3> three{};
+    return many ? (vec ? rows(three, wide) : rows(three, scalar))
+                : (vec ? rows(two, wide) : rows(two, scalar));
+  }
 }
 
 template <class T, class RT>

@@ -13,9 +13,11 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# x-lines of 255, 256, 257, 258 and 516 pairs, even and odd; one line; ragged
+# x-lines of 255, 256, 257, 258 and 516 pairs, even and odd; one line; ragged; and
+# classes of more than 100,000 pairs, even and odd
 GRIDS = [(510, 3, 3, 1), (511, 2, 3, 1), (512, 4, 2, 2), (514, 4, 4, 2), (1031, 3, 2, 1),
-         (1032, 2, 2, 2), (513, 1, 1, 1), (34, 6, 10, 2), (256, 2, 6, 2)]
+         (1032, 2, 2, 2), (513, 1, 1, 1), (34, 6, 10, 2), (256, 2, 6, 2),
+         (130, 101, 100, 1), (131, 101, 101, 1)]
 
 
 def view(a, odd):
