@@ -894,7 +894,8 @@ __device__ __forceinline__ void prefetch_lines(const LevelMat<VT> &A, const Clas
 // line no values of a second row: one form for everything but FORM_WIDE, with a
 // test for left-out entries at every term, took 1475 us for the symmetric FP64
 // sweep at 255^3 (1190 so; with one row per thread 1601) and 640 for the BF16 one
-// (460; 512), 6849 from vectors off the boundary at 384^3 (5380 before the pairs).
+// (460; 512); from vectors off the boundary FP64 1586 at 258 x 200 x 200 (1172;
+// 1053), BF16 2556 at 384^3 (1430; 1590).
 // Against one row per thread with a second load phase for the second colour
 // (before) the pair issues all its loads once: FP64, HBM-bound, the symmetric
 // sweep at 256^3 takes 1186 us = 6.1 TB/s of 8 B per nonzero and pass (before,
@@ -1853,14 +1854,50 @@ constexpr int64_t kManyPairs = 100000;
 // block would be shorter (lines of 192, 96 and 48 pairs, 384^3: 5630 against
 // 5611).  A class of few lines takes fewer lines per block so that there is a
 // block for each SM twice over (a launch is then bound by one block's latency).
+// Lines longer than that (FP64: of more than 128 pairs) go a block each, in chunks.
+// Their sweep takes one round of chunks after another, as many as waves of blocks
+// times chunks of a line, whatever the block's size, for the registers keep the
+// warps of an SM to the same number (FP64 8, BF16 with three blocks of 256 per SM
+// 24).  FP64 takes 128 threads, or the one of 256 and 64 that saves a twentieth of
+// the rounds and more; BF16 256, or 160 or 192 for a fifth.  Symmetric FP64 sweep,
+// us, with 64 / 128 / 256 threads (one row per thread, before the pairs): 258 x 200
+// x 200 876 / 1071 / 1159 (1054), 514 x 128 x 128 697 / 753 / 958 (905), 700 x 100 x
+// 100 612 / 574 / 680 (789), 2048 x 64 x 64 702 / 702 / 666 (1012), 700 x 32 x 32 123
+// / 95 / 106 (130); 384^3 3857 with 64, 4480 with 192 (5359); from a view at an odd
+// element 514 x 128 x 128 709 / 763 / 1009 (902), 384^3 3955 with 64 (5380).  BF16, 256 / 192 / 160: 514 x 128 x 128 327 / 289 / 283 (339), at an odd
+// element 367 / 324 / 317 (340), 1026 x 64 x 64 181 / 159 / 174 (194), 3000 x 50 x 50
+// 316 / 320 / 345 (340).
 struct GsBlock {
   int lines, threads;
 };
+int64_t gs_rounds(const ClassInfo &C, int threads, int per_sm) {
+  const int64_t waves = (C.lines + 148 * per_sm - 1) / (148 * per_sm);
+  return waves * ((C.len[0] + threads - 1) / threads);
+}
+template <class T>
+int chunk_threads(const ClassInfo &C) {
+  constexpr bool fp64 = std::is_same<T, double>::value;
+  struct { int threads, per_sm; } const size[2][3] = {{{256, 3}, {160, 5}, {192, 4}},
+                                                      {{128, 2}, {256, 1}, {64, 4}}};
+  const auto &s = size[fp64];
+  int best = 0;
+  int64_t most = 0;   // rounds that a size may take to be chosen
+  for (int i = 0; i < 3; ++i) {
+    const int64_t r = gs_rounds(C, s[i].threads, s[i].per_sm);
+    if (i > 0 && r > most) continue;
+    best = i;
+    most = i > 0 ? r - 1 : fp64 ? r * 19 / 20 : r * 4 / 5;
+  }
+  return s[best].threads;
+}
 template <class T>
 GsBlock gs_block(const ClassInfo &C) {
   const int len = C.len[0];
+  constexpr bool fp64 = std::is_same<T, double>::value;
+  if (fp64 ? len > 128 : len > kThreads && (int64_t)C.lines * len > kManyPairs)
+    return {1, std::min(chunk_threads<T>(C), (len + 31) / 32 * 32)};
   const bool fills = (int64_t)C.lines * len > kManyPairs && 128 / len * len >= 120;
-  const int target = std::is_same<T, double>::value || fills ? 128 : kThreads;
+  const int target = fp64 || fills ? 128 : kThreads;
   const int lines = std::min(std::max(1, target / len), std::max(1, C.lines / (2 * 148)));
   return {lines, std::min(kThreads, (lines * len + 31) / 32 * 32)};
 }

@@ -13,11 +13,13 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# x-lines of 255, 256, 257, 258 and 516 pairs, even and odd; one line; ragged; and
-# classes of more than 100,000 pairs, even and odd
+# x-lines of 255, 256, 257, 258 and 516 pairs, even and odd; one line; ragged;
+# classes of more than 100,000 pairs, even and odd; many long lines, in chunks of
+# 64 (FP64; BF16 one chunk), 128 (256), 64 (160) and 64 (192) pairs
 GRIDS = [(510, 3, 3, 1), (511, 2, 3, 1), (512, 4, 2, 2), (514, 4, 4, 2), (1031, 3, 2, 1),
          (1032, 2, 2, 2), (513, 1, 1, 1), (34, 6, 10, 2), (256, 2, 6, 2),
-         (130, 101, 100, 1), (131, 101, 101, 1)]
+         (130, 101, 100, 1), (131, 101, 101, 1),
+         (384, 48, 48, 1), (700, 32, 32, 1), (514, 64, 64, 1), (1025, 46, 46, 1)]
 
 
 def view(a, odd):
