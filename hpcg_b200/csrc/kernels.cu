@@ -728,7 +728,8 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
     const int t = (DIR == 0 ? chunks - 1 - ch : ch) * nb + tid;
     const bool act = t < cnt;
     PairId id;
-    RowVals<VT> ve, vo{};
+    RowVals<VT> ve, vo;
+    if (FORM != FORM_WIDE) vo = RowVals<VT>{};   // (the wide form loads it always)
     uint32_t oe = 0u, oo = 0u;
     T xl[5][4];
     T se = T(0), so = T(0), ax = T(0), xe = T(0), xo = T(0), re = T(0);
@@ -1864,9 +1865,10 @@ constexpr int64_t kManyPairs = 100000;
 // x 200 876 / 1071 / 1159 (1054), 514 x 128 x 128 697 / 753 / 958 (905), 700 x 100 x
 // 100 612 / 574 / 680 (789), 2048 x 64 x 64 702 / 702 / 666 (1012), 700 x 32 x 32 123
 // / 95 / 106 (130); 384^3 3857 with 64, 4480 with 192 (5359); from a view at an odd
-// element 514 x 128 x 128 709 / 763 / 1009 (902), 384^3 3955 with 64 (5380).  BF16, 256 / 192 / 160: 514 x 128 x 128 327 / 289 / 283 (339), at an odd
-// element 367 / 324 / 317 (340), 1026 x 64 x 64 181 / 159 / 174 (194), 3000 x 50 x 50
-// 316 / 320 / 345 (340).
+// element 514 x 128 x 128 709 / 763 / 1009 (902), 384^3 3955 with 64 (5380).  BF16,
+// 256 / 192 / 160: 514 x 128 x 128 327 / 289 / 283 (339), at an odd element 367 / 324
+// / 317 (340), 1026 x 64 x 64 181 / 159 / 174 (194), 3000 x 50 x 50 316 / 320 / 345
+// (340).
 struct GsBlock {
   int lines, threads;
 };
