@@ -1675,6 +1675,13 @@ static int vector_blocks(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * (n > (1 << 23) ? 8 : 4)));
 }
 
+// Blocks of k_dot, which writes nothing: five per SM where the vectors stream from
+// HBM, at 512^3 335 us a call (eight: 357; one element per thread, before the tiles:
+// 338), at 384^3 172 (184; 171), at 256^3 84 (85; 85).
+static int dot_blocks(int64_t n) {
+  return n > (1 << 23) ? std::min(vector_blocks(n), 148 * 5) : vector_blocks(n);
+}
+
 // Blocks of the kernels that take one element per thread and step (k_copy,
 // k_copy_z, k_cg_xflush; with a reduction k_absmax_diff, k_cg_init), four elements
 // a thread at least.  They have a quarter of a tiled kernel's loads under way and
@@ -2053,7 +2060,7 @@ int launch_waxpby(int64_t n, double alpha, const double *x, double beta, const d
 int launch_dot(int64_t n, const double *x, const double *y, const Reduce &red, double *out,
                cudaStream_t s) {
   by_width([&](auto wide) {
-    k_dot<wide.value><<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, red, FIN_STORE, out, nullptr);
+    k_dot<wide.value><<<dot_blocks(n), kThreads, 0, s>>>(n, x, y, red, FIN_STORE, out, nullptr);
   }, x, y);
   return 1;
 }
@@ -2061,7 +2068,7 @@ int launch_dot(int64_t n, const double *x, const double *y, const Reduce &red, d
 int launch_dot_finish(int64_t n, const double *x, const double *y, const Reduce &red, int fin,
                       CgState *st, cudaStream_t s) {
   by_width([&](auto wide) {
-    k_dot<wide.value><<<vector_blocks(n), kThreads, 0, s>>>(n, x, y, red, fin, st, &st->done);
+    k_dot<wide.value><<<dot_blocks(n), kThreads, 0, s>>>(n, x, y, red, fin, st, &st->done);
   }, x, y);
   return 1;
 }

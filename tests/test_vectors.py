@@ -1,6 +1,7 @@
 """The vector kernels at the edges of their tiles (1024 elements, four per
-thread) and of the grid (592 blocks, 1184 above 2^23 elements; 1024 for the
-residual), with vectors on and off a two-element boundary: WAXPBY bit-exact in its three branches
+thread) and of the grid (592 blocks, above 2^23 elements 1184 and 740 for the dot
+product; 1024 for the residual), with vectors on and off a two-element
+boundary: WAXPBY bit-exact in its three branches
 (src/ComputeWAXPBY_ref.cpp:52-67), in place as well; dot products
 (src/ComputeDotProduct_ref.cpp:48-63) to 1e-13 of the exactly rounded sum of
 products, the same bits wherever the vectors start; the residual exact.
@@ -14,7 +15,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 # more than 2^23 elements: the larger grid, at its edge and with several tiles a block
-LARGE = [1 << 23, (1 << 23) + 1, 1184 * 1024 * 8 - 1, 1184 * 1024 * 8 + 513]
+LARGE = [1 << 23, (1 << 23) + 1, 740 * 1024 * 12 + 1, 1184 * 1024 * 8 - 1,
+         1184 * 1024 * 8 + 513]
 SIZES = [1, 2, 255, 1023, 1024, 1025, 2047, 2051, 592 * 1024 - 1, 592 * 1024 + 1,
          1024 * 1024 - 1, 1024 * 1024 + 1, 1184 * 1024 + 513]
 
@@ -69,7 +71,7 @@ def test_large_vectors(large, n):
     x, y, w = (torch.empty(n + 2, dtype=torch.float64, device="cuda").uniform_(-1, 1, generator=g)
                for _ in range(3))
     hx, hy = x.cpu().numpy(), y.cpu().numpy()
-    # sums of at most n / (1184 * 256) + 1 products a thread, and of the threads'
+    # sums of at most n / (740 * 256) + 1 products a thread, and of the threads'
     want = float(np.sum(hx[:n].astype(np.longdouble) * hy[1:n + 1]))
     bound = 1e-13 * float(np.abs(hx[:n] * hy[1:n + 1]).sum())
     got = large.dot(x[:n], y[1:n + 1])
