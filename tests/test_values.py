@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dims,levels", [((1, 1, 1), 1), ((3, 1, 2), 1), ((5, 7, 3), 1), ((64, 2, 2), 2),
                                          ((65, 3, 2), 1), ((33, 9, 5), 1), ((16, 24, 8), 4),
-                                         ((130, 6, 4), 2)])
+                                         ((130, 6, 4), 2), ((1, 40, 30), 1), ((130, 1, 4), 1),
+                                         ((70, 33, 1), 1), ((1, 1, 200), 1)])
 def test_values(dims, levels):
     from hpcg_b200 import Problem
     nx, ny, nz = dims
