@@ -70,7 +70,7 @@ struct ClassInfo {
   int lines;        // lines of this class
   int len[2];       // rows per line for px = 0 / 1
   int64_t start[2]; // storage row of the first row of colour 2q+px
-  FastDiv dlen[2];  // division by len[px]
+  FastDiv dlen;     // division by len[0]
   FastDiv dnyq;     // division by nyq
 };
 

@@ -48,8 +48,8 @@ struct GenMat {
 // The entries of a storage row, kChunk at a time: their columns and values are
 // loaded together and then their x entries together, so that a row waits for
 // memory twice per chunk and not twice per entry (the sums keep the row's own
-// order).  Padding entries up to the slice's width hold value 0 and column 0;
-// they are loaded but not added.  Rows of up to 27 entries are one chunk.
+// order).  The padding up to the slice's width (value 0, column 0) is not read.
+// Rows of up to 27 entries are one chunk.
 constexpr int kChunk = 27;
 struct GenRow {
   int m = 0;          // entries; 0: no row

@@ -478,13 +478,12 @@ __device__ __forceinline__ void store2(float *p, float u, float v) {
   *reinterpret_cast<float2 *>(p) = make_float2(u, v);
 }
 
-// x[2i-1 .. 2i+2] on line l into v[0..3]; what does not exist (or is not on)
-// reads as 0, the value its slots hold, so that the product drops out whatever
+// x[2i-1 .. 2i+2] on line l into v[0..3]; what does not exist reads as 0, the value its slots hold, so that the product drops out whatever
 // x holds elsewhere.  vec: the two middle entries with one load (x and nx allow it).
 template <class VT, class T>
 __device__ __forceinline__ void load_line(const LevelMat<VT> &A, const PairId &id, const T *xr,
-                                          int l, bool on, bool vec, T *v, int site) {
-  bool ok = on && has_line(id, l);
+                                          int l, bool vec, T *v, int site) {
+  bool ok = has_line(id, l);
   const T *q = xr + A.off[3 * l + 1];
 #ifdef HPCGX_CHECKED
   if (ok && !line_inside(A, id, vec, l)) {
@@ -582,7 +581,7 @@ k_spmv(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ ClassSet 
           load_vals(A.vals, id.ko, p, NeedAll(), vo);
         }
 #pragma unroll
-        for (int i = 0; i < 3; ++i) load_line(A, id, xr, 3 * p + i, true, vec, v[i], 2);
+        for (int i = 0; i < 3; ++i) load_line(A, id, xr, 3 * p + i, vec, v[i], 2);
 #pragma unroll
         for (int s = 0; s < 9; ++s) {
           se = term_add(oe, 9 * p + s, se, ve[s], v[s / 3][s % 3]);
@@ -695,7 +694,6 @@ __device__ __forceinline__ T gs_tail(uint32_t out, int c, const V &val, const T 
 // the pair was issued before the first update.
 // ZERO: x is zero for the colours above and for the row itself (first forward
 //       sweep after ZeroVector); their terms are skipped at compile time.
-//       zero: the same at run time, those entries read as 0.
 // pro:  colour 0 first receives the prolongated coarse correction -- except in
 //       the first plane of a slab with a halo below, whose correction is added
 //       before the halo exchange (the slab below reads that plane).
@@ -713,7 +711,7 @@ __device__ __forceinline__ T gs_tail(uint32_t out, int c, const V &val, const T 
 // its second row must see updated updated.
 template <int DIR, bool ZERO, bool SYM3, bool AHEAD, int FORM, class VT, class T, class RT>
 __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo &C, int ce, int j0,
-                                         int j1, bool zero, bool pro, bool res, bool vec,
+                                         int j1, bool pro, bool res, bool vec,
                                          const uint32_t *left_out, const RT *r, T *x, const T *xc,
                                          T *rc, T *sh, const int *done) {
   const int cnt = (j1 - j0) * C.len[0];
@@ -777,7 +775,7 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
           if (ZERO && !there)
             to[0] = to[1] = to[2] = to[3] = T(0);
           else
-            load_line(A, id, xr, l, !zero || there, vec, to, 4);
+            load_line(A, id, xr, l, vec, to, 4);
         }
         se = gs_head<0, ZERO>(oe, ce, ve, xh, re);
         so = gs_head<1, ZERO>(oo, co, vo, xh, ro);
@@ -856,7 +854,7 @@ __device__ __forceinline__ void gs_pairs(const LevelMat<VT> &A, const ClassInfo 
       for (int p = 0; p < 3; ++p) ve.load(A.vals, id.ke, p, NeedAll());
 #pragma unroll
       for (int l = 0; l < 9; ++l)
-        load_line(A, id, (const T *)x + id.row, l, true, vec,
+        load_line(A, id, (const T *)x + id.row, l, vec,
                   l < 4 ? xh[l < 4 ? l : 0] : xl[l < 4 ? 0 : l - 4], 4);
       const uint32_t oe = left_out ? left_out[id.ke] : 0u;
       const T sum = gs_head<0, false>(oe, ce, ve, xh, vec_to(r[id.row], T()));
@@ -925,7 +923,7 @@ k_gs_class(const __grid_constant__ LevelMat<VT> A, const __grid_constant__ Class
     if (jn < jend) prefetch_lines(A, C, jn, min(jn + lpb, jend));
   }
   gs_pairs<DIR, ZERO, (MODE & GS_SYM3) != 0, MINB != 3, FORM>(
-      A, C, 2 * (Q >= 0 ? Q : C.q), j0, min(j0 + lpb, jend), false, (MODE & GS_PROLONG) != 0,
+      A, C, 2 * (Q >= 0 ? Q : C.q), j0, min(j0 + lpb, jend), (MODE & GS_PROLONG) != 0,
       (MODE & GS_RESTRICT) != 0, is_wide<FORM>(vec), FORM == FORM_HOLES ? A.left_out : nullptr, r, x,
       xc, rc, sh, done);
 }
@@ -1742,8 +1740,7 @@ void plan_level(LevelDev &L, int nx, int ny, int nz) {
     C.len[1] = nx / 2;
     C.start[0] = L.cstart[2 * q];
     C.start[1] = L.cstart[2 * q + 1];
-    C.dlen[0] = make_fastdiv((uint32_t)C.len[0]);
-    C.dlen[1] = make_fastdiv((uint32_t)C.len[1]);
+    C.dlen = make_fastdiv((uint32_t)C.len[0]);
     C.dnyq = make_fastdiv((uint32_t)C.nyq);
     L.spmv_blocks += (int)(((int64_t)C.lines * C.len[0] + kThreads - 1) / kThreads);
   }

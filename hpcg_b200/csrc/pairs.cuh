@@ -25,7 +25,7 @@ __host__ __device__ __forceinline__ PairId pair_at(const LevelMat<VT> &A, const 
                                                    int j0, int t) {
   PairId id;
   const int Le = C.len[0];
-  const int jl = (int)fdiv((uint32_t)t, C.dlen[0]);
+  const int jl = (int)fdiv((uint32_t)t, C.dlen);
   id.pos = t - jl * Le;
   const int j = j0 + jl;
   const int jz = (int)fdiv((uint32_t)j, C.dnyq);

@@ -63,8 +63,8 @@ int main(int, char **argv) {
       C.len[px] = (nx - px + 1) / 2;
       C.start[px] = A.srows;
       A.srows += ((int64_t)C.lines * C.len[px] + 31) / 32 * 32;
-      C.dlen[px] = make_fastdiv((uint32_t)C.len[px]);
     }
+    C.dlen = make_fastdiv((uint32_t)C.len[0]);
     C.dnyq = make_fastdiv((uint32_t)C.nyq);
   }
   const int vecs = nx % 2 == 0 ? 2 : 1;   // two-element accesses need even lines
