@@ -286,9 +286,9 @@ def run_kernels(args):
     y = torch.empty_like(u)
     u32 = u.float()
     ops = {
-        "spmv": (lambda: P.spmv(u, y=y), 12 * nnz + 16 * n),
-        "spmv_stencil": (lambda: P.spmv(u, y=y, stencil_cols=True), 8 * nnz + 16 * n),
-        "symgs": (lambda: P.symgs(v, x), 24 * nnz + 48 * n),
+        "spmv": (lambda: P.spmv(u, y=y), 8 * nnz + 16 * n),
+        # seven class launches: three quarters of the rows twice, the last class once
+        "symgs": (lambda: P.symgs(v, x), 14 * nnz + 42 * n),
         "dot": (lambda: P.dot(u, v), 16 * n),
         "waxpby": (lambda: P.waxpby(0.7, u, -1.3, v, w=y), 24 * n),
         "spmv_bf16": (lambda: P.spmv_mixed(u32), 2 * nnz + 8 * n),
@@ -615,26 +615,6 @@ def main():
     x_diff = gnorm(x_mixed - x64) / gnorm(x64)
     err_u = gnorm(x_mixed - u) / gnorm(u)
 
-    # ---------------- FP64 after asking for the mixed solver's column derivation
-    # (every FP64 operator derives its columns, so this is the solve above)
-    P.set_stencil_columns(True)
-    solve(False)
-    t64s = []
-    for _ in range(max(1, args.fp64_steps)):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        with torch.cuda.stream(stream):
-            e0.record(stream)
-        k64s, nr64s, nr064s = solve(False)
-        with torch.cuda.stream(stream):
-            e1.record(stream)
-        torch.cuda.synchronize()
-        t64s.append(e0.elapsed_time(e1) * 1e-3)
-    t_fp64s = statistics.mean(t64s)
-    x64s_diff = gnorm(x - x64) / gnorm(x64)
-    if not sharded:
-        ib["fp64_stencil_cols"] = P.iteration_bytes(CG_MG)
-    P.set_stencil_columns(False)
-
     # ---------------- end to end through the C ABI from pinned host buffers:
     # b copied in and x copied out inside each timed solve
     bh = b.cpu().pin_memory()
@@ -651,8 +631,7 @@ def main():
     t_e2e = statistics.mean(te2e)
 
     # ---------------- max over ranks
-    t_mixed, t_fp64, t_fp64s, t_e2e = max_over_ranks([t_mixed, t_fp64, t_fp64s, t_e2e], dist,
-                                                     f"cuda:{dev}")
+    t_mixed, t_fp64, t_e2e = max_over_ranks([t_mixed, t_fp64, t_e2e], dist, f"cuda:{dev}")
 
     flops, b64, b32, n0, z0 = model(dims)
     peak, peak_kind = peaks()
@@ -707,12 +686,6 @@ def main():
         "iterations": {"mixed": iters_mixed[-1], "fp64": k64},
         "fp64_time_s": t_fp64,
         "speedup_mixed_vs_fp64": t_fp64 / t_mixed,
-        "fp64_stencil_cols_time_s": t_fp64s,
-        "speedup_mixed_vs_fp64_stencil_cols": t_fp64s / t_mixed,
-        "fp64_stencil_cols": {"iterations": k64s, "x_rel_diff_vs_fp64": x64s_diff,
-                              "note": "FP64 PCG with every column derived from the stencil "
-                                      "offsets, as the mixed solver does: the mixed-vs-FP64 "
-                                      "ratio from precision alone"},
         "fp64_rel_residual": {"mixed_recursive": relres_mixed, "mixed_true": true_mixed,
                               "fp64_true": true_fp64},
         "x_rel_diff_vs_fp64": x_diff, "x_rel_err_vs_u": err_u,
@@ -720,7 +693,6 @@ def main():
         "roofline_iteration": {
             "mixed": whole_iteration("mixed", iters_mixed[-1], t_mixed),
             "fp64": whole_iteration("fp64", k64, t_fp64),
-            "fp64_stencil_cols": whole_iteration("fp64_stencil_cols", k64s, t_fp64s),
             "model": "this implementation's algorithmic bytes per CG iteration "
                      "(hpcgx_iteration_bytes: every launch of the iteration, real nonzeros, each "
                      "vector element once per launch) x iterations / solve time"},

@@ -3,7 +3,7 @@ odd grids, one rank and sharded, and no kernel may meet an out-of-range
 storage row, vector row or column (libhpcgx_checked.so records the first one
 and redirects the access into the buffers or leaves it out;
 hpcgx_check_status reports it; test_pair_index.py checks that answer).
-This stands in for a memory checker, which this GPU pool does not run.
+This stands in for a memory checker.
 The checked library is loaded in a child process (HPCGX_LIBRARY=checked is
 read when the library is first loaded)."""
 import os
@@ -18,6 +18,8 @@ from conftest import ROOT
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(16, 16, 16), (24, 24, 24), (16, 24, 32), (64, 32, 16)]
+# one level: odd and flat grids, smaller than a vector access's reach, lines in chunks
+ODD = [(1, 1, 1), (2, 1, 1), (3, 1, 2), (9, 7, 5), (33, 1, 4), (1, 6, 5), (515, 3, 2), (131, 101, 101)]
 
 
 def _run(rank, out):
@@ -54,6 +56,44 @@ def _run(rank, out):
         check_status()
         done.append(("one rank", dims))
         P.close()
+    for dims in ODD:
+        P = Problem(*dims, levels=1)
+        P.generate("hpcg")
+        P.build_mixed()
+        n = P.rows()
+        # vectors on and off a two-element boundary
+        for odd in (0, 1):
+            u, b = (P.fill_uniform(s, -1.0, 1.0, n=n + 1)[odd:n + odd] for s in (1, 2))
+            u32 = torch.cat([u.float()] * 2)[odd:n + odd]
+            P.spmv(u)
+            P.spmv_mixed(u32)
+            P.symgs(b, u)
+            P.symgs_mixed(b, u32)
+            P.mg(b)
+            P.mg_mixed(b)
+            P.cg(b, u, 1, 0.0)
+            P.cg_mixed(b, u, 1, 0.0)
+        v, _ = P.get_values()
+        P.set_values(v.reshape(-1))
+        P.adjoint_grad(u.clone(), b.clone())
+        check_status()
+        done.append(("one level", dims))
+        P.close()
+    # rows that leave out entries
+    P = Problem(4, 3, 2, levels=1)
+    n = P.rows()
+    cols = np.tile(np.arange(n, dtype=np.int32)[:, None], (1, 27))
+    vals = np.zeros((n, 27))
+    vals[:, 0] = 26.0
+    P.load_level(0, np.ones(n, np.uint8), cols.reshape(-1), vals.reshape(-1))
+    u, b = P.fill_uniform(1, -1.0, 1.0), P.fill_uniform(2, -1.0, 1.0)
+    assert torch.equal(P.spmv(u), 26.0 * u)
+    P.symgs(b, u)
+    P.cg(b, u, 1, 0.0)
+    P.adjoint_grad(u, b)
+    check_status()
+    done.append(("left out", (4, 3, 2)))
+    P.close()
     # variable coefficients and the adjoint gradient
     from hpcg_b200 import varcoef_problem
     P, vals = varcoef_problem(16, 16, 16, seed=2, sigma=0.5)
@@ -93,4 +133,4 @@ def test_checked_build_meets_no_bad_index():
     mgr = mp.get_context("spawn").Manager()
     out = mgr.dict()
     mp.start_processes(_run, args=(out,), nprocs=1, join=True, start_method="spawn")
-    assert len(out["done"]) == len(GRIDS) + 3
+    assert len(out["done"]) == len(GRIDS) + len(ODD) + 4

@@ -153,9 +153,9 @@ def test_against_reference_golden(oracle):
 
 
 def test_fp64_stencil_columns(grid, oracle):
-    """hpcgx_set_stencil_columns: the FP64 operators with every column derived
-    from the stencil offsets give the same bits as with the stored columns
-    (SpMV, SYMGS on every level, the V-cycle) and CG_ref's iteration count."""
+    """hpcgx_set_stencil_columns changes nothing: every operator derives its columns
+    from the stencil offsets (SpMV, SYMGS on every level and the V-cycle bit for
+    bit, CG_ref's iteration count), and a solve has the same bits on and off."""
     from hpcg_b200 import Problem
     L, b, xe, _ = setup(grid, oracle)
     P = Problem(*grid)
@@ -175,13 +175,10 @@ def test_fp64_stencil_columns(grid, oracle):
         k, nr, nr0 = P.cg(cuda(b), x, 500, 1e-10)
         _, ok, _, _ = oracle.cg(L, b, np.zeros(n), 500, 1e-10, coloured=True)
         assert k == ok and nr / nr0 <= 1e-10
-        # and back to the stored columns: the rebuilt iteration graph agrees (the
-        # stencil-column SpMV takes two line groups per block, so its fused p.Ap
-        # sums its partials in another order: norms agree to 1e-6, not bitwise)
         P.set_stencil_columns(False)
-        x.zero_()
-        k2, nr2, _ = P.cg(cuda(b), x, 500, 1e-10)
-        assert k2 == k and abs(nr2 / nr - 1) < 1e-6
+        y = torch.zeros(n, dtype=torch.float64, device="cuda")
+        assert P.cg(cuda(b), y, 500, 1e-10) == (k, nr, nr0)
+        assert torch.equal(x, y)
     finally:
         P.close()
 
