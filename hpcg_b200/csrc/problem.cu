@@ -1077,22 +1077,17 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
     pending[h] = false;
     const int64_t c1 = std::min(slices, c0 + kPinnedSlices);
     const int64_t k0 = c0 * HPCGX_SLICE, e0 = c0 * kSliceElems;
+    std::fill(bo, bo + (c1 - c0) * HPCGX_SLICE, 0u);
     parallel_for((c1 - c0) * HPCGX_SLICE, [&](int64_t a, int64_t e, int t) {
       for (int64_t k = k0 + a; k < k0 + e; ++k) {
         int ix, iy, iz;
         const int64_t row = natural_row_host(A, k, ix, iy, iz);
-        uint32_t has = 0u;
         auto blank = [&]() {
           for (int s = 0; s < HPCGX_STENCIL; ++s) bv[vidx(k, s) - e0] = 0.0;
-          has = 0u;
         };
         blank();
-        bo[k - k0] = 0u;
         if (row < 0) continue;   // padding
-        auto put = [&](int s, double v) {
-          bv[vidx(k, s) - e0] = v;
-          has |= 1u << s;
-        };
+        auto put = [&](int s, double v) { bv[vidx(k, s) - e0] = v; };
         if (!fast_row(row, ix, iy, iz, put)) {
           blank();
           if (!scan_row(row, put).empty()) {
@@ -1100,10 +1095,15 @@ int load_level_impl(hpcgx_problem *p, int level, Nnz nnz_of, Get get) {
             return;
           }
         }
-        const uint32_t out = ~has & stencil_bits(ix > 0, ix + 1 < A.nx, iy > 0, iy + 1 < A.ny,
-                                                 iz > 0, iz + 1 < A.nz);
-        bo[k - k0] = out;
-        if (out) gone.store(true, std::memory_order_relaxed);
+        const bool xm = ix > 0, xp = ix + 1 < A.nx, ym = iy > 0, yp = iy + 1 < A.ny, zm = iz > 0,
+                   zp = iz + 1 < A.nz;
+        if (nnz_of(row) < (1 + xm + xp) * (1 + ym + yp) * (1 + zm + zp)) {
+          // an existing neighbour without an entry: which
+          uint32_t has = 0u;
+          scan_row(row, [&](int s, double) { has |= 1u << s; });
+          bo[k - k0] = ~has & stencil_bits(xm, xp, ym, yp, zm, zp);
+          gone.store(true, std::memory_order_relaxed);
+        }
       }
     });
     for (char f : bad) failed |= f != 0;
