@@ -114,8 +114,11 @@ int hpcgx_set_diagonal_host(hpcgx_problem *p, int level, const double *diag_host
 int hpcgx_get_diagonal_host(hpcgx_problem *p, int level, double *diag_host);
 /* Level values in natural row order, 27 stencil slots per row
  * (slot (dz+1)*9+(dy+1)*3+(dx+1)); device pointers.  set_values ignores
- * slots without a neighbour; with recoarsen != 0 the coarse levels are
- * rebuilt from the new finest values (variable-coefficient rule). */
+ * slots without a neighbour and stores every other one, so that no row leaves
+ * out an entry afterwards; with recoarsen != 0 the coarse levels are rebuilt from
+ * the new finest values (variable-coefficient rule).  cols27: the neighbour, or
+ * the row itself where a slot has none or a loaded row leaves the entry out (a
+ * stored 0 keeps its column). */
 int hpcgx_set_values(hpcgx_problem *p, int level, const double *vals27, int recoarsen);
 int hpcgx_get_values(hpcgx_problem *p, int level, double *vals27, int32_t *cols27);
 /* Device memory held by the problem (OptimizeProblemMemoryUse,
